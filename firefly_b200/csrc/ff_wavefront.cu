@@ -60,8 +60,11 @@ constexpr uint32_t PH_START = 0, PH_FLIGHT = 1, PH_DONE = 2, PH_DRAINED = 3;
 constexpr uint64_t kDefaultPoolTarget = 1ull << 23;
 
 // Counter words of one frame (zeroed at the start of each frame); one block
-// of kCtrStride words per frame parity.
-enum { C_EXT = 0, C_SH = 1, C_MAT = 2, C_ACTIVE = 2 + kKinds, C_WORDS = 8 + kKinds };
+// of kCtrStride words per frame parity.  C_EXT: extension rays of the frame,
+// all of them counted by k_logic (its camera rays, C_CAM, and one
+// continuation per queued vertex); C_SH: shadow rays; C_MAT + k: vertices of
+// material kind k.
+enum { C_EXT = 0, C_SH = 1, C_MAT = 2, C_ACTIVE = 2 + kKinds, C_CAM = 3 + kKinds, C_WORDS = 8 + kKinds };
 constexpr uint32_t kCtrStride = 32;
 
 // The slot's ray (origin, direction) and its visibility word: byte k = the
@@ -166,7 +169,7 @@ struct WF {
     uint32_t* sh_tag;    // per queued shadow ray: the byte of its answer (vis_byte, or 4 * slot + k in vis2)
     uint32_t* mat_queue;   // kKinds * P
     uint32_t* ctr;         // C_WORDS
-    unsigned long long* totals;  // [0] extension rays, [1] shadow rays, [2] samples
+    unsigned long long* totals;  // [0] extension rays, [1] shadow rays of the frames reset so far
     // scene
     const FFShadeTri* shade;
     const FFTangentTri* tan;   // tangent frames, or null when no material has a normal texture
@@ -207,18 +210,15 @@ __device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v
 __device__ __forceinline__ float4 f4(float3 v, float w = 0.f) { return make_float4(v.x, v.y, v.z, w); }
 
 // Warp-aggregated append (the reference's atomicAggInc, kernel.cu:24-36, on
-// *_sync intrinsics): one atomic per warp and per queue.
-__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want, unsigned long long* total)
+// *_sync intrinsics): one atomic per warp.
+__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want)
 {
     const uint32_t mask = __ballot_sync(__activemask(), want);
     if (!want) return 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t leader = __ffs(mask) - 1;
     uint32_t base = 0;
-    if (lane == leader) {
-        base = atomicAdd(counter, (uint32_t)__popc(mask));
-        if (total) atomicAdd(total, (unsigned long long)__popc(mask));
-    }
+    if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(mask));
     base = __shfl_sync(mask, base, leader);
     return base + __popc(mask & ((1u << lane) - 1u));
 }
@@ -286,8 +286,9 @@ __device__ __forceinline__ bool consume_pending(const WF& w, uint32_t s, float4&
 // ADJ: the path-replay adjoint's instantiation (the slot's sum holds the
 // current sample's radiance only, in plain FP32 adds as the megakernel
 // adjoint sums it; no film).
+constexpr int kLogicBlock = 256;
 template <bool ADJ>
-__global__ void __launch_bounds__(256) k_logic(WF w)
+__global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     bool push_ext = false;
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(256) k_logic(WF w)
                 }
             }
             if (!ADJ && w.cache_mode) {
-                const uint32_t qi = warp_append(w.n_queries, query, nullptr);
+                const uint32_t qi = warp_append(w.n_queries, query);
                 if (query) w.queries[qi] = rec;
             }
         } else if (!ADJ && w.defer && ph == PH_DONE) {
@@ -521,19 +522,52 @@ __global__ void __launch_bounds__(256) k_logic(WF w)
             w.phase[s] = PH_DRAINED;
         }
     }
-    // compaction into the extension queue and the material queues
-    const uint32_t qe = warp_append(&w.ctr[C_EXT], push_ext, &w.totals[0]);
-    if (push_ext) {
-        w.ext_rays[qe] = ray;
-        w.ext_tag[qe] = s;
-    }
+    // Compaction into the camera-ray part of the extension queue and the
+    // material queues, one atomic per block and queue.  Every counter sits in
+    // one L2 line, whose atomics run one after the other; with one atomic per
+    // warp and queue, and a 64-bit running total beside each, k_logic took
+    // 87.2 ms of the 1.3M-triangle 64-spp step, 76.9 ms so (with k_shade's
+    // single append per warp the step went from 259.7 to 249.0 ms, the small
+    // room's 256 x 256 x 16 from 3.06 to 2.87 ms).
+    constexpr int kQ = kKinds + 2;   // the kinds, camera rays, active slots
+    __shared__ uint32_t s_n[kLogicBlock / 32][kQ], s_base[kQ];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const int my_q = kind >= 0 ? kind : (push_ext ? kKinds : -1);   // a slot enters at most one queue
+    uint32_t before = 0;   // lanes below in the same queue
 #pragma unroll
-    for (int k = 0; k < kKinds; ++k) {
-        const uint32_t qm = warp_append(&w.ctr[C_MAT + k], kind == k, nullptr);
-        if (kind == k) w.mat_queue[(size_t)k * w.P + qm] = s;
+    for (int q = 0; q < kQ; ++q) {
+        const uint32_t mask = __ballot_sync(0xffffffffu, q <= kKinds ? my_q == q : active);
+        if (my_q == q) before = __popc(mask & ((1u << lane) - 1u));
+        if (lane == 0) s_n[warp][q] = (uint32_t)__popc(mask);
     }
-    const uint32_t am = __ballot_sync(0xffffffffu, active);
-    if ((threadIdx.x & 31u) == 0 && am) atomicAdd(&w.ctr[C_ACTIVE], (uint32_t)__popc(am));
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        uint32_t sum = 0;
+        if (threadIdx.x < kQ) {
+#pragma unroll
+            for (int v = 0; v < kLogicBlock / 32; ++v) {
+                const uint32_t n = s_n[v][threadIdx.x];
+                s_n[v][threadIdx.x] = sum;
+                sum += n;
+            }
+        }
+        const uint32_t ext = __reduce_add_sync(0xffffffffu, threadIdx.x <= kKinds ? sum : 0u);
+        if (threadIdx.x < kQ && sum) {
+            const int c = threadIdx.x < kKinds ? C_MAT + (int)threadIdx.x : (threadIdx.x == kKinds ? C_CAM : C_ACTIVE);
+            s_base[threadIdx.x] = atomicAdd(&w.ctr[c], sum);
+        }
+        if (threadIdx.x == kQ && ext) atomicAdd(&w.ctr[C_EXT], ext);
+    }
+    __syncthreads();
+    if (my_q >= 0) {
+        const uint32_t pos = s_base[my_q] + s_n[warp][my_q] + before;
+        if (kind >= 0) {
+            w.mat_queue[(size_t)kind * w.P + pos] = s;
+        } else {
+            w.ext_rays[pos] = ray;
+            w.ext_tag[pos] = s;
+        }
+    }
     if (ADJ) {
         touched = __reduce_add_sync(0xffffffffu, touched);
         touched_r = __reduce_add_sync(0xffffffffu, touched_r);
@@ -557,6 +591,10 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
     // every lane runs the same number of iterations so the queue appends can use full-warp ballots
     const uint32_t iters = (n + stride - 1) / stride;
     const uint32_t base = blockIdx.x * blockDim.x + threadIdx.x;
+    // every queued vertex continues with one extension ray: their places
+    // follow the camera rays', kind after kind in queue order
+    uint32_t ext_base = w.ctr[C_CAM];
+    for (int k = 0; k < KIND; ++k) ext_base += w.ctr[C_MAT + k];
     LightCtx lc;
     if (!SEL) lc = select_light(w.lights, 0u, 0u);   // the fixed light
     for (uint32_t it = 0; it < iters; ++it) {
@@ -630,29 +668,20 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
                 w.v_albedo[s] = f4(mat.albedo, __uint_as_float(flags));
             }
         }
-        const uint32_t qe = warp_append(&w.ctr[C_EXT], valid, &w.totals[0]);
-        if (valid) {
-            w.ext_rays[qe] = make_ext_ray(o.ext_o, o.ext_d, ext_two);
-            w.ext_tag[qe] = s;
-        }
-        const uint32_t q0 = warp_append(&w.ctr[C_SH], o.ray_nee, &w.totals[1]);
-        const uint32_t q1 = warp_append(&w.ctr[C_SH], o.ray_spec, &w.totals[1]);
-        const uint32_t q2 = warp_append(&w.ctr[C_SH], o.ray_diff, &w.totals[1]);
+        // one append for the warp's shadow rays of all three sorts; its answer is
+        // needed only after the writes below
+        const uint32_t m0 = __ballot_sync(0xffffffffu, o.ray_nee), m1 = __ballot_sync(0xffffffffu, o.ray_spec),
+                       m2 = __ballot_sync(0xffffffffu, o.ray_diff);
+        const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+        const uint32_t n0 = __popc(m0), n1 = __popc(m1), n2 = __popc(m2);
+        uint32_t sh_base = 0;
+        if (lane == 0 && n0 + n1 + n2) sh_base = atomicAdd(&w.ctr[C_SH], n0 + n1 + n2);
         // answer tags: bytes of the slot's vis word in SlotRay, or of its word in vis2 (deferred mode)
         const bool defer = !ADJ && w.defer;
-        if (o.ray_nee) {
-            w.sh_rays[q0] = o.r_nee;
-            w.sh_tag[q0] = defer ? 4u * s : vis_byte(s, 0);
-        }
-        if (o.ray_spec) {
-            w.sh_rays[q1] = o.r_spec;
-            w.sh_tag[q1] = defer ? 4u * s + 1u : vis_byte(s, 1);
-        }
-        if (o.ray_diff) {
-            w.sh_rays[q2] = o.r_diff;
-            w.sh_tag[q2] = defer ? 4u * s + 2u : vis_byte(s, 2);
-        }
         if (valid) {
+            const uint32_t qe = ext_base + qi;
+            w.ext_rays[qe] = make_ext_ray(o.ext_o, o.ext_d, ext_two);
+            w.ext_tag[qe] = s;
             // the continuation ray and the queued-rays byte, one whole record
             const uint32_t queued = ((o.ray_nee ? 1u : 0u) | (o.ray_spec ? 2u : 0u) | (o.ray_diff ? 4u : 0u)) << 24;
             w.ray[s] = SlotRay{o.ext_o.x, o.ext_o.y, o.ext_o.z, queued, o.ext_d.x, o.ext_d.y, o.ext_d.z, 0.f};
@@ -665,6 +694,21 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
                 pq[2] = f4(o.c_spec);
                 pq[3] = f4(o.c_diff);
             }
+        }
+        sh_base = __shfl_sync(0xffffffffu, sh_base, 0);
+        const uint32_t q0 = sh_base + __popc(m0 & below), q1 = sh_base + n0 + __popc(m1 & below),
+                       q2 = sh_base + n0 + n1 + __popc(m2 & below);
+        if (o.ray_nee) {
+            w.sh_rays[q0] = o.r_nee;
+            w.sh_tag[q0] = defer ? 4u * s : vis_byte(s, 0);
+        }
+        if (o.ray_spec) {
+            w.sh_rays[q1] = o.r_spec;
+            w.sh_tag[q1] = defer ? 4u * s + 1u : vis_byte(s, 1);
+        }
+        if (o.ray_diff) {
+            w.sh_rays[q2] = o.r_diff;
+            w.sh_tag[q2] = defer ? 4u * s + 2u : vis_byte(s, 2);
         }
     }
 }
@@ -720,13 +764,23 @@ __global__ void k_resolve(WF w, float4* __restrict__ film_acc, float4* __restric
     film_n[p] = n;
 }
 
-__global__ void k_reset_counters(uint32_t* ctr, unsigned long long* trace_counters)
+// Adds the rays of the last frame that used these counters to the totals
+// (extension, shadow) and clears the counters for the next one.
+__global__ void k_reset_counters(uint32_t* ctr, unsigned long long* trace_counters, unsigned long long* totals)
 {
+    if (threadIdx.x < 2) {
+        totals[threadIdx.x] += ctr[threadIdx.x == 0 ? C_EXT : C_SH];
+        trace_counters[threadIdx.x] = 0ull;
+    }
+    __syncthreads();
     if (threadIdx.x < C_WORDS) ctr[threadIdx.x] = 0;
-    if (threadIdx.x < 2) trace_counters[threadIdx.x] = 0ull;
 }
 
 }  // namespace
+
+// Byte offsets of the control block's parts (each carved to a 256-byte boundary).
+constexpr size_t kCtlTotals = 256, kCtlErr = 512, kCtlFetch = 1024, kCtlBytes = 1280;
+static_assert(2 * kCtrStride * sizeof(uint32_t) == kCtlTotals, "two parities' counter words fill the first part");
 
 // Per-film workspace: slot arrays and queues, reused while the pool size is unchanged.
 struct FFWavefrontWS {
@@ -746,7 +800,25 @@ struct FFWavefrontWS {
     ff_ray* sh_rays_base[2] = {nullptr, nullptr};
     uint32_t* sh_tag_base[2] = {nullptr, nullptr};
     unsigned long long* fetch = nullptr;      // profiled renders: nodes / tris of the closest, then the any-hit traces
-    uint32_t* h_active = nullptr;             // pinned host word for the frame-loop check
+    // the counter words, totals, error count, trace counters and fetch counts
+    // are carved one after the other (kCtlBytes from ctr_base): one memset
+    // clears them, one copy brings them to this pinned block
+    char* h_ctl = nullptr;
+    // extension ([0]) and shadow ([1]) rays of the call, from h_ctl: the
+    // totals of the frames reset so far and the counters of the last ones
+    uint64_t host_rays(int k) const
+    {
+        const uint32_t* c = reinterpret_cast<const uint32_t*>(h_ctl);
+        const uint64_t* t = reinterpret_cast<const uint64_t*>(h_ctl + kCtlTotals);
+        const int word = k == 0 ? C_EXT : C_SH;
+        return t[k] + c[word] + c[kCtrStride + word];
+    }
+    unsigned int host_err() const { return *reinterpret_cast<const unsigned int*>(h_ctl + kCtlErr); }
+    const unsigned long long* host_fetch() const
+    {
+        return reinterpret_cast<const unsigned long long*>(h_ctl + kCtlFetch);
+    }
+    uint32_t* h_active() const { return reinterpret_cast<uint32_t*>(h_ctl); }
     // the any-hit trace runs on `side` beside the closest-hit trace: its
     // blocks take the SMs the closest-hit trace's finished blocks leave
     cudaStream_t side = nullptr;
@@ -770,7 +842,7 @@ struct FFWavefrontWS {
     }
     ~FFWavefrontWS()
     {
-        if (h_active) cudaFreeHost(h_active);
+        if (h_ctl) cudaFreeHost(h_ctl);
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         for (int i = 0; i < 2; ++i)
@@ -883,6 +955,7 @@ void ws_setup(FFWavefrontWS* ws, uint32_t P)
     ws->err = carve<unsigned int>(p, 4);
     ws->trace_ctr = carve<unsigned long long>(p, 4);
     ws->fetch = carve<unsigned long long>(p, 4);
+    if (!ws->h_ctl) FF_CUDA_CHECK(cudaMallocHost(&ws->h_ctl, kCtlBytes));
     ws->sh_rays_base[1] = nullptr;
     ws->sh_tag_base[1] = nullptr;
     w.pend = nullptr;
@@ -966,9 +1039,7 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     std::vector<ff_material> mats(scene->num_materials);
     FF_CUDA_CHECK(cudaMemcpyAsync(mats.data(), scene->materials.ptr, sizeof(ff_material) * mats.size(),
                                   cudaMemcpyDeviceToHost, stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(unsigned long long), stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(ws->err, 0, sizeof(unsigned int), stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(ws->fetch, 0, 4 * sizeof(unsigned long long), stream));
+    FF_CUDA_CHECK(cudaMemsetAsync(ws->ctr_base, 0, kCtlBytes, stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(stream));
     bool kind_used[kKinds] = {false, false, false, false, false};
     for (auto& mt : mats) kind_used[mt.kind] = true;
@@ -995,9 +1066,8 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     };
     uint32_t frames = 0;
     uint32_t active = 1;
-    if (!ws->h_active) FF_CUDA_CHECK(cudaMallocHost(&ws->h_active, sizeof(uint32_t)));
     ws->ensure_streams();
-    uint32_t* h_active = ws->h_active;
+    uint32_t* h_active = ws->h_active();
     const uint32_t max_frames = (st->spp + 1) * (st->max_depth + 2) + 8;
     // Deferred light terms (every render but the cached one): the any-hit
     // trace of frame f runs on the side stream beside k_logic, k_shade and
@@ -1022,9 +1092,9 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
             unsigned long long* tctr = ws->trace_ctr + 2 * par;
             uint8_t* occ = defer ? reinterpret_cast<uint8_t*>(w.vis2 + (size_t)par * P) : reinterpret_cast<uint8_t*>(w.ray);
             if (defer && !profile && frames >= 2) FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[par], 0));
-            k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, tctr);
+            k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, tctr, w.totals);
             mark();
-            k_logic<false><<<(P + 255) / 256, 256, 0, stream>>>(w);
+            k_logic<false><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
             mark();
             // with stage timing (profile) every launch stays on the one stream
             FFWavefrontWS* side = profile ? nullptr : ws;
@@ -1094,13 +1164,10 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
                                                    film->count.as<uint32_t>());
     FF_CUDA_CHECK(cudaGetLastError());
     FF_CUDA_CHECK(cudaEventRecord(ctx->ev1, stream));
-    unsigned long long totals[3] = {0, 0, 0}, fetch[4] = {0, 0, 0, 0};
-    unsigned int err = 0;
-    FF_CUDA_CHECK(cudaMemcpyAsync(totals, w.totals, sizeof(totals), cudaMemcpyDeviceToHost, stream));
-    FF_CUDA_CHECK(cudaMemcpyAsync(&err, ws->err, sizeof(err), cudaMemcpyDeviceToHost, stream));
-    if (profile) FF_CUDA_CHECK(cudaMemcpyAsync(fetch, ws->fetch, sizeof(fetch), cudaMemcpyDeviceToHost, stream));
+    FF_CUDA_CHECK(cudaMemcpyAsync(ws->h_ctl, ws->ctr_base, kCtlBytes, cudaMemcpyDeviceToHost, stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-    if (err) throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
+    const unsigned long long* fetch = ws->host_fetch();
+    if (ws->host_err()) throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
     if (stats) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -1129,8 +1196,8 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
         // per frame: counter reset, logic, one shade per kind, two traces
         // (+ two counting passes when profiled); init and resolve; the flush
         stats->kernel_launches = frames * (4u + (uint32_t)n_kinds + (profile ? 2u : 0u)) + 2u + (defer ? 2u : 0u);
-        stats->extension_rays = totals[0];
-        stats->shadow_rays = totals[1];
+        stats->extension_rays = ws->host_rays(0);
+        stats->shadow_rays = ws->host_rays(1);
         stats->samples = (uint64_t)st->spp * WH;
         stats->frames = frames;
         stats->ms_total = ms;
@@ -1230,8 +1297,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     std::vector<ff_material> mats(scene->num_materials);
     FF_CUDA_CHECK(cudaMemcpyAsync(mats.data(), scene->materials.ptr, sizeof(ff_material) * mats.size(),
                                   cudaMemcpyDeviceToHost, stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(unsigned long long), stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(ws->err, 0, sizeof(unsigned int), stream));
+    FF_CUDA_CHECK(cudaMemsetAsync(ws->ctr_base, 0, kCtlBytes, stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(stream));
     bool kind_used[kKinds] = {false, false, false, false, false};
     for (auto& mt : mats) kind_used[mt.kind] = true;
@@ -1253,16 +1319,15 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     };
     uint32_t frames = 0;
     uint32_t active = 1;
-    if (!ws->h_active) FF_CUDA_CHECK(cudaMallocHost(&ws->h_active, sizeof(uint32_t)));
     ws->ensure_streams();
-    uint32_t* h_active = ws->h_active;
+    uint32_t* h_active = ws->h_active();
     // two passes per sample
     const uint32_t max_frames = 2 * (st->spp + 1) * (st->max_depth + 2) + 8;
     while (active && frames < max_frames) {
         for (int b = 0; b < 4; ++b) {
-            k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, ws->trace_ctr);
+            k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, ws->trace_ctr, w.totals);
             mark();
-            k_logic<true><<<(P + 255) / 256, 256, 0, stream>>>(w);
+            k_logic<true><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
             mark();
             // side streams as in ff_wavefront_render (one stream under stage timing)
             launch_shade<false, true, true>(w, kind_used, shade_blocks, stream, profile ? nullptr : ws);
@@ -1293,12 +1358,9 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
         active = *h_active;
     }
     if (active) throw FFError{FF_ERR_INTERNAL, "wavefront adjoint did not finish within its frame bound"};
-    unsigned long long totals[2] = {0, 0};
-    unsigned int err = 0;
-    FF_CUDA_CHECK(cudaMemcpyAsync(totals, w.totals, sizeof(totals), cudaMemcpyDeviceToHost, stream));
-    FF_CUDA_CHECK(cudaMemcpyAsync(&err, ws->err, sizeof(err), cudaMemcpyDeviceToHost, stream));
+    FF_CUDA_CHECK(cudaMemcpyAsync(ws->h_ctl, ws->ctr_base, kCtlBytes, cudaMemcpyDeviceToHost, stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-    if (err) throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
+    if (ws->host_err()) throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
     if (profile) {
         // 5 marks per frame: logic | shade | trace extension | trace shadow
         float t[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1317,8 +1379,8 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     for (auto e : evs) cudaEventDestroy(e);
     if (stats) {
         stats->kernel_launches = frames * (4u + (uint32_t)n_kinds) + 1u;   // counter reset, logic, shades, traces; init
-        stats->extension_rays = totals[0];
-        stats->shadow_rays = totals[1];
+        stats->extension_rays = ws->host_rays(0);
+        stats->shadow_rays = ws->host_rays(1);
         stats->frames = frames;
     }
 }
