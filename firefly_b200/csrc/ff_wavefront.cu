@@ -48,9 +48,10 @@ namespace {
 using namespace ffp;
 using namespace ffadj;
 constexpr int kKinds = 5;
+// WF::state: the phase in the low two bits, the path length above them.
 // PH_DRAINED (deferred mode): finished, and the last pending light terms
 // added, so later frames skip the slot without reading its records.
-constexpr uint32_t PH_START = 0, PH_FLIGHT = 1, PH_DONE = 2, PH_DRAINED = 3;
+constexpr uint32_t PH_FLIGHT = 1, PH_DONE = 2, PH_DRAINED = 3, kPhaseBits = 2;
 
 // Path-pool size when ff_render_settings.max_paths is 0: m slots per pixel,
 // m = min(spp, this / (w*h)), at least 1.  Measured on the 1.3M-triangle
@@ -103,7 +104,7 @@ struct __align__(32) SlotVtx {
 // rays queued.  Indexed [frame parity][slot].
 struct __align__(32) SlotPend {
     float bx, by, bz;
-    uint32_t stamp;   // frame + kStampBase of the shading; any other value: nothing pending
+    uint32_t stamp;   // WF::stamp0 + frame of the shading; any other value: nothing pending
     float nee_x, nee_y, nee_z;
     uint32_t queued;  // bit k: shadow ray k was queued
     float spec_x, spec_y, spec_z, pad0;
@@ -112,14 +113,16 @@ struct __align__(32) SlotPend {
 static_assert(sizeof(SlotRay) == 32 && sizeof(SlotShade) == 32 && sizeof(SlotMis) == 32 && sizeof(SlotVtx) == 64 &&
                   sizeof(SlotPend) == 64,
               "slot records are whole 32-byte sectors");
-constexpr uint32_t kStampBase = 16;
+// Stamps never repeat over the renders of a workspace (stamp0 grows), so
+// records left by an earlier render need no clearing; 0 marks a fresh record.
+constexpr uint32_t kFirstStamp = 16;
 // Deferred mode: blocks per SM of the any-hit trace (its persistent grid, of
 // 8 that fit), leaving the rest of each SM to k_logic and k_shade of the next
 // frame.  Measured on the 1.3M-triangle scene at 64 spp: 3 blocks 262.7 ms
 // per step, 4: 265.4-266.0, 5: 268.7, 6: 272.7; later, against 256.3-256.4
 // with 3: 2 blocks 267.4-267.6, 1: 298.2 (the trace then outlasts the next
 // frame, whose successor waits for it).
-constexpr int kDeferShadowBlocks = 3;   // stamps of real frames are >= 16; 0 marks an empty record
+constexpr int kDeferShadowBlocks = 3;
 constexpr uint32_t kVtxMatBits = 24, kVtxLenShift = 24, kVtxLenMask = 0x7f;
 // Byte of shadow ray k's answer for slot s in the SlotRay array (the tag the
 // any-hit trace writes to): the low three bytes of the vis word.
@@ -134,13 +137,13 @@ struct WF {
     uint32_t seed, max_depth, rr_depth, mode;
     int32_t light;
     float shadow_offset;
+    uint32_t spp, sample_offset;
+    uint32_t first;   // 1 in a render's first frame: every slot starts, whatever its state holds
     // slot state
-    uint32_t* samples_left;
     uint32_t* next_sample;
     uint32_t* key;
-    uint32_t* length;
-    uint32_t* phase;
-    float4* beta;
+    uint32_t* state;
+    float4* beta;     // throughput; deferred mode: that after the last vertex (k_shade), w = 1 if the path ends there
     // Per-slot records that k_shade reaches through its material queue, i.e.
     // scattered over the slots: each is whole 32-byte sectors, so a scattered
     // access moves no bytes it does not use (a lone 16-byte field fetches or
@@ -152,13 +155,12 @@ struct WF {
     float4* hit_ngeo;     // interpolated normal, written only under a normal texture
     float4* acc;
     float4* acc_c;
-    uint32_t* cnt;
     // deferred light terms (defer = 1): the frame's parity and number, the
     // pending records and the any-hit answers (byte k of a slot's word: shadow
     // ray k occluded), both [2][P]; the shadow queue and the frame counters
     // are per parity too, so that the any-hit trace of frame f runs beside
     // k_logic and k_shade of frame f + 1
-    uint32_t defer, par, frame;
+    uint32_t defer, par, frame, stamp0;
     SlotPend* pend;
     uint32_t* vis2;
     // queues
@@ -234,19 +236,18 @@ __device__ __forceinline__ void kahan_add(float4& sum, float4& c, float3 x)
 __device__ __forceinline__ uint32_t slot_pixel(const WF& w, uint32_t s) { return s % w.WH; }
 
 // wf_generate + dCamera::gen_ray for slot s, sample `sample`.
-__device__ void start_sample(const WF& w, uint32_t s, uint32_t sample, bool& push, ff_ray& ray)
+__device__ __forceinline__ void start_sample(const WF& w, uint32_t s, uint32_t sample, ff_ray& ray)
 {
     const uint32_t pix = slot_pixel(w, s);
     const uint32_t key = ff_path_key(w.seed, pix, sample);
     w.key[s] = key;
-    w.length[s] = 0;
+    w.state[s] = PH_FLIGHT;
     w.beta[s] = make_float4(1.f, 1.f, 1.f, 0.f);
     const int x = (int)(pix % w.W), y = (int)(pix / w.W);
     float3 o, d;
     gen_camera_ray(w.cam, (int)w.W, (int)w.H, x, y, rand2(key, 0, DIM_CAM_JITTER), rand2(key, 0, DIM_CAM_LENS), o, d);
     w.ray[s] = SlotRay{o.x, o.y, o.z, 0u, d.x, d.y, d.z, 0.f};
     ray = ff_ray{o.x, o.y, o.z, 0.f, d.x, d.y, d.z, __int_as_float(0x7f800000)};
-    push = true;
 }
 
 // Deferred mode: the light terms of the vertex slot s shaded two frames ago
@@ -259,7 +260,7 @@ __device__ __forceinline__ bool consume_pending(const WF& w, uint32_t s, float4&
     const size_t i = (size_t)w.par * w.P + s;
     const float4* pq = reinterpret_cast<const float4*>(w.pend + i);
     const float4 a = pq[0];
-    if (__float_as_uint(a.w) != w.frame + kStampBase - 2u) return false;
+    if (__float_as_uint(a.w) != w.stamp0 + w.frame - 2u) return false;
     const float4 b = pq[1];
     const uint32_t q = __float_as_uint(b.w);
     const uint32_t vw = w.vis2[i];
@@ -283,6 +284,12 @@ __device__ __forceinline__ bool consume_pending(const WF& w, uint32_t s, float4&
     return true;
 }
 
+// Whether a vertex's BSDF sample carries nothing on, which ends the path.
+__device__ __forceinline__ bool path_ends(float3 f, float pdf)
+{
+    return f == make_float3(0.f, 0.f, 0.f) || pdf == 0.f;
+}
+
 // ADJ: the path-replay adjoint's instantiation (the slot's sum holds the
 // current sample's radiance only, in plain FP32 adds as the megakernel
 // adjoint sums it; no film).
@@ -291,32 +298,37 @@ template <bool ADJ>
 __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    bool push_ext = false;
-    ff_ray ray{};
+    bool push_ext = false;   // the slot starts sample `sample`
+    uint32_t sample = 0;
     int kind = -1;
     bool active = false;
     uint32_t touched = 0, touched_r = 0;
     if (s < w.P) {
-        uint32_t ph = w.phase[s];
-        if (ph == PH_START) {
-            const uint32_t smp = w.next_sample[s];
-            w.next_sample[s] = smp + w.m;
-            start_sample(w, s, smp, push_ext, ray);
-            w.phase[s] = PH_FLIGHT;
-            if (ADJ) {
-                w.pass[s] = 0;
-                w.acc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint32_t state = w.first ? 0u : w.state[s];
+        const uint32_t ph = state & ((1u << kPhaseBits) - 1u);
+        if (w.first) {
+            const uint32_t lane = s / w.WH;   // which of the m slots of its pixel
+            w.acc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ADJ) w.pass[s] = 0;
+            else w.acc_c[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (lane < w.spp) {
+                sample = w.sample_offset + lane;
+                w.next_sample[s] = sample + w.m;
+                push_ext = true;
+                active = true;
+            } else {
+                w.state[s] = PH_DRAINED;
             }
-            active = true;
         } else if (ph == PH_FLIGHT) {
             active = true;
             const uint32_t key = w.key[s];
             const ff_hit hit = w.ext_hits[s];
-            const uint32_t L = w.length[s] + 1;  // wf_extend's length++
+            const uint32_t L = (state >> kPhaseBits) + 1;  // wf_extend's length++
             const bool found = hit.prim != -1;
             const SlotRay sr = w.ray[s];
             const float3 ro = make_float3(sr.ox, sr.oy, sr.oz), rd = make_float3(sr.dx, sr.dy, sr.dz);
-            float3 beta = xyz(w.beta[s]);
+            const float4 beta4 = w.beta[s];
+            float3 beta = xyz(beta4);
             float4 acc = w.acc[s];
             float4 accc = ADJ ? make_float4(0.f, 0.f, 0.f, 0.f) : w.acc_c[s];   // no compensation in the adjoint
             if (!ADJ && w.defer) consume_pending(w, s, acc, accc);
@@ -347,8 +359,12 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                 }
             }
             if (L > 1) {
-                const SlotShade sd = w.shd[s];
-                if (ADJ || !w.defer) {   // (deferred light terms were added above)
+                bool ends;   // the vertex's BSDF sample carries nothing on
+                if (!ADJ && w.defer) {
+                    // light terms were added above; k_shade left the throughput after the vertex
+                    ends = beta4.w != 0.f;
+                } else {
+                    const SlotShade sd = w.shd[s];
                     // kernel.cu:357-359: light_brdf * beta when the NEE ray was unoccluded
                     const uint32_t vw = sr.vis;
                     const bool vis = (vw & (1u << 24)) && !(vw & 0xffu);
@@ -410,14 +426,13 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                         }
                         kahan_add(acc, accc, lb * beta);
                     }
+                    const float3 f = make_float3(sd.f_x, sd.f_y, sd.f_z);
+                    ends = path_ends(f, sd.pdf);
+                    if (!ends) beta *= (f * sd.cosine) / sd.pdf;
                 }
-                const float3 f = make_float3(sd.f_x, sd.f_y, sd.f_z);
-                const float pdf = sd.pdf;
-                const float cosine = sd.cosine;
-                if (f == make_float3(0.f, 0.f, 0.f) || pdf == 0.f) {
+                if (ends) {
                     terminate = true;
                 } else {
-                    beta *= (f * cosine) / pdf;
                     if (L > w.rr_depth) {
                         const float q_rr = hmax(0.05f, 1.f - beta.y);
                         if (ff_rand(key, dim_of(L, DIM_RR)) < q_rr) terminate = true;
@@ -466,8 +481,9 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                     // Light sample (kernel.cu:435, light get_direction).
                     float3 wi, sp;
                     sample_light(select_light(w.lights, key, L), pos, key, L, wi, sp);
-                    w.length[s] = L;
-                    w.beta[s] = f4(beta);
+                    w.state[s] = PH_FLIGHT | L << kPhaseBits;
+                    // (deferred mode: it still holds the throughput, unless the roulette scaled it)
+                    if (ADJ || !w.defer || L > w.rr_depth) w.beta[s] = f4(beta);
                     SlotVtx vx;
                     vx.px = pos.x, vx.py = pos.y, vx.pz = pos.z;
                     vx.word = t.material | (L << kVtxLenShift) | (back ? kBackFace : 0u);
@@ -488,21 +504,19 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                     w.l_total[s] = acc;
                     w.pass[s] = 1u;
                     w.acc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    start_sample(w, s, w.next_sample[s] - w.m, push_ext, ray);
+                    sample = w.next_sample[s] - w.m;
+                    push_ext = true;
                 } else {
-                    w.cnt[s] += 1u;
-                    const uint32_t left = w.samples_left[s] - 1u;
-                    w.samples_left[s] = left;
+                    sample = w.next_sample[s];
                     if (ADJ) {
                         w.pass[s] = 0u;
                         w.acc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
                     }
-                    if (left > 0) {
-                        const uint32_t smp = w.next_sample[s];
-                        w.next_sample[s] = smp + w.m;
-                        start_sample(w, s, smp, push_ext, ray);
+                    if (sample - w.sample_offset < w.spp) {
+                        w.next_sample[s] = sample + w.m;
+                        push_ext = true;
                     } else {
-                        w.phase[s] = PH_DONE;
+                        w.state[s] = PH_DONE;
                         active = false;
                     }
                 }
@@ -519,9 +533,11 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                 w.acc[s] = acc;
                 w.acc_c[s] = accc;
             }
-            w.phase[s] = PH_DRAINED;
+            w.state[s] = PH_DRAINED;
         }
     }
+    ff_ray ray{};
+    if (push_ext) start_sample(w, s, sample, ray);
     // Compaction into the camera-ray part of the extension queue and the
     // material queues, one atomic per block and queue.  Every counter sits in
     // one L2 line, whose atomics run one after the other; with one atomic per
@@ -604,7 +620,6 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
         o.ray_nee = o.ray_spec = o.ray_diff = false;
         bool ext_two = false;   // the continuation runs inside an object: traced two-sided
         uint32_t s = 0;
-        float4 beta_v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (valid) {
             s = w.mat_queue[(size_t)KIND * w.P + qi];
             const SlotVtx vx = w.vtx[s];
@@ -641,7 +656,8 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
             if (w.mode == FF_MODE_CORRECTED || KIND == FF_MAT_DIELECTRIC || back)
                 o.ext_o = pos + ng * (side * w.shadow_offset);
             ext_two = runs_inside(back, KIND == FF_MAT_DIELECTRIC, side);
-            w.shd[s] = SlotShade{o.c_nee.x, o.c_nee.y, o.c_nee.z, o.ext_pdf, o.ext_f.x, o.ext_f.y, o.ext_f.z, o.ext_cos};
+            if (ADJ || !w.defer)
+                w.shd[s] = SlotShade{o.c_nee.x, o.c_nee.y, o.c_nee.z, o.ext_pdf, o.ext_f.x, o.ext_f.y, o.ext_f.z, o.ext_cos};
             // the kinds with BSDF-sampled light terms (deferred mode: in the pending record)
             if ((KIND == FF_MAT_MIX || KIND == FF_MAT_DIELECTRIC) && (ADJ || !w.defer))
                 w.mis[s] = SlotMis{o.c_spec.x, o.c_spec.y, o.c_spec.z, 0.f, o.c_diff.x, o.c_diff.y, o.c_diff.z, 0.f};
@@ -687,12 +703,24 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
             w.ray[s] = SlotRay{o.ext_o.x, o.ext_o.y, o.ext_o.z, queued, o.ext_d.x, o.ext_d.y, o.ext_d.z, 0.f};
             if (defer) {
                 // the light terms with the throughput they multiply, for k_logic two frames on
-                beta_v = w.beta[s];   // the throughput at this vertex
+                const float4 beta_v = w.beta[s];   // the throughput at this vertex
                 float4* pq = reinterpret_cast<float4*>(w.pend + (size_t)w.par * w.P + s);
-                pq[0] = make_float4(beta_v.x, beta_v.y, beta_v.z, __uint_as_float(w.frame + kStampBase));
+                pq[0] = make_float4(beta_v.x, beta_v.y, beta_v.z, __uint_as_float(w.stamp0 + w.frame));
                 pq[1] = make_float4(o.c_nee.x, o.c_nee.y, o.c_nee.z, __uint_as_float(queued >> 24));
                 pq[2] = f4(o.c_spec);
                 pq[3] = f4(o.c_diff);
+                // and the throughput after it in the place of the one before: 16
+                // bytes of a sector just read, where its factors took a record of
+                // 32 here and 32 more to read in k_logic.  With that, the sample
+                // counts derived from next_sample and no pass that clears the
+                // slots before the first frame, the 1.3M-triangle 64-spp step
+                // went from 234.4 to 230.5 ms, the inverse step (512 x 512 x 16)
+                // from 15.9 to 14.9 ms; more warps per SM (smaller blocks, fewer
+                // registers) change neither, so k_logic follows its bytes.
+                const bool ends = path_ends(o.ext_f, o.ext_pdf);
+                float3 beta = xyz(beta_v);
+                if (!ends) beta *= (o.ext_f * o.ext_cos) / o.ext_pdf;
+                w.beta[s] = f4(beta, ends ? 1.f : 0.f);
             }
         }
         sh_base = __shfl_sync(0xffffffffu, sh_base, 0);
@@ -710,26 +738,6 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
             w.sh_rays[q2] = o.r_diff;
             w.sh_tag[q2] = defer ? 4u * s + 2u : vis_byte(s, 2);
         }
-    }
-}
-
-__global__ void k_init(WF w, uint32_t spp, uint32_t sample_offset)
-{
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= w.P) return;
-    if (w.pass) w.pass[s] = 0u;
-    const uint32_t lane = s / w.WH;  // which of the m slots of its pixel
-    const uint32_t left = lane < spp ? (spp - lane + w.m - 1) / w.m : 0u;
-    w.samples_left[s] = left;
-    w.next_sample[s] = sample_offset + lane;
-    w.phase[s] = left ? PH_START : PH_DONE;
-    w.acc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    w.acc_c[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    w.cnt[s] = 0;
-    w.ray[s].vis = 0u;
-    if (w.defer) {
-        w.pend[s].stamp = 0u;
-        w.pend[(size_t)w.P + s].stamp = 0u;
     }
 }
 
@@ -752,16 +760,14 @@ __global__ void k_resolve(WF w, float4* __restrict__ film_acc, float4* __restric
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= w.WH) return;
     float4 sum = film_acc[p], c = film_c[p];
-    uint32_t n = film_n[p];
     for (uint32_t k = 0; k < w.m; ++k) {
         const uint32_t s = p + k * w.WH;
         const float4 a = w.acc[s], ac = w.acc_c[s];
         kahan_add(sum, c, make_float3(a.x - ac.x, a.y - ac.y, a.z - ac.z));
-        n += w.cnt[s];
     }
     film_acc[p] = sum;
     film_c[p] = c;
-    film_n[p] = n;
+    film_n[p] += w.spp;
 }
 
 // Adds the rays of the last frame that used these counters to the totals
@@ -789,6 +795,7 @@ struct FFWavefrontWS {
     DevBuf adj_buf;   // the adjoint's per-slot arrays (allocated by ff_wavefront_adjoint only)
     DevBuf defer_buf; // the deferred light terms' arrays (allocated by ff_render only)
     uint32_t defer_P = 0;
+    uint64_t next_stamp = kFirstStamp;   // the first stamp the next render may use
     uint32_t adj_P = 0;
     WF w{};
     unsigned int* err = nullptr;
@@ -912,9 +919,9 @@ size_t ws_bytes(uint32_t P)
 {
     size_t b = 0;
     auto add = [&](size_t s, size_t n) { b += (s * n + 255) & ~size_t(255); };
-    add(4, P) /*samples_left*/; add(4, P); add(4, P); add(4, P); add(4, P);
+    add(4, P) /*next_sample*/; add(4, P) /*key*/; add(4, P) /*state*/;
     add(16, P) /*beta*/; add(sizeof(SlotRay), P); add(sizeof(SlotShade), P); add(sizeof(SlotMis), P);
-    add(sizeof(SlotVtx), P); add(16, P) /*hit_ngeo*/; add(16, P); add(16, P) /*acc, acc_c*/; add(4, P) /*cnt*/;
+    add(sizeof(SlotVtx), P); add(16, P) /*hit_ngeo*/; add(16, P); add(16, P) /*acc, acc_c*/;
     add(sizeof(ff_ray), P); add(4, P); add(sizeof(ff_hit), P); add(sizeof(ff_ray), 3ull * P); add(4, 3ull * P);
     add(4, (size_t)kKinds * P); add(4, 2 * kCtrStride); add(8, 8); add(4, 4); add(8, 4); add(8, 4);
     return b;
@@ -929,11 +936,9 @@ void ws_setup(FFWavefrontWS* ws, uint32_t P)
     char* p = ws->buf.as<char>();
     WF& w = ws->w;
     w.P = P;
-    w.samples_left = carve<uint32_t>(p, P);
     w.next_sample = carve<uint32_t>(p, P);
     w.key = carve<uint32_t>(p, P);
-    w.length = carve<uint32_t>(p, P);
-    w.phase = carve<uint32_t>(p, P);
+    w.state = carve<uint32_t>(p, P);
     w.beta = carve<float4>(p, P);
     w.ray = carve<SlotRay>(p, P);
     w.shd = carve<SlotShade>(p, P);
@@ -942,7 +947,6 @@ void ws_setup(FFWavefrontWS* ws, uint32_t P)
     w.hit_ngeo = carve<float4>(p, P);
     w.acc = carve<float4>(p, P);
     w.acc_c = carve<float4>(p, P);
-    w.cnt = carve<uint32_t>(p, P);
     w.ext_rays = carve<ff_ray>(p, P);
     w.ext_tag = carve<uint32_t>(p, P);
     w.ext_hits = carve<ff_hit>(p, P);
@@ -950,7 +954,7 @@ void ws_setup(FFWavefrontWS* ws, uint32_t P)
     ws->sh_tag_base[0] = w.sh_tag = carve<uint32_t>(p, 3ull * P);
     w.mat_queue = carve<uint32_t>(p, (size_t)kKinds * P);
     ws->ctr_base = w.ctr = carve<uint32_t>(p, 2 * kCtrStride);
-    w.defer = w.par = w.frame = 0u;
+    w.defer = w.par = w.frame = w.first = 0u;
     w.totals = carve<unsigned long long>(p, 8);
     ws->err = carve<unsigned int>(p, 4);
     ws->trace_ctr = carve<unsigned long long>(p, 4);
@@ -967,7 +971,7 @@ void ws_setup(FFWavefrontWS* ws, uint32_t P)
 // The deferred light terms' arrays (ff_render only, allocated on its first
 // call for this pool size): the second frame parity's shadow queue, the
 // pending records and the answer words of both parities.
-void defer_setup(FFWavefrontWS* ws, uint32_t P)
+void defer_setup(FFWavefrontWS* ws, uint32_t P, cudaStream_t stream)
 {
     if (ws->defer_P == P && ws->defer_buf.ptr) return;
     size_t b = 0;
@@ -982,6 +986,8 @@ void defer_setup(FFWavefrontWS* ws, uint32_t P)
     ws->sh_tag_base[1] = carve<uint32_t>(p, 3ull * P);
     ws->w.pend = carve<SlotPend>(p, 2ull * P);
     ws->w.vis2 = carve<uint32_t>(p, 2ull * P);
+    FF_CUDA_CHECK(cudaMemsetAsync(ws->w.pend, 0, sizeof(SlotPend) * 2ull * P, stream));
+    ws->next_stamp = kFirstStamp;
     ws->defer_P = P;
 }
 
@@ -1010,6 +1016,8 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     w.W = film->width;
     w.H = film->height;
     w.m = m;
+    w.spp = st->spp;
+    w.sample_offset = st->sample_offset;
     w.seed = st->seed;
     w.max_depth = st->max_depth;
     w.rr_depth = st->rr_depth;
@@ -1046,11 +1054,20 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
 
     // deferred light terms: every render but the cached one (see the frame loop)
     const bool defer = hook == nullptr;
-    if (defer) defer_setup(ws, P);
     w.defer = defer ? 1u : 0u;
+    const uint32_t max_frames = (st->spp + 1) * (st->max_depth + 2) + 8;
     FF_CUDA_CHECK(cudaEventRecord(ctx->ev0, stream));
-    k_init<<<(P + 255) / 256, 256, 0, stream>>>(w, st->spp, st->sample_offset);
-    FF_CUDA_CHECK(cudaGetLastError());
+    if (defer) {
+        defer_setup(ws, P, stream);
+        // stamps of frames 0, 1, ... of this render, two above the last one's
+        // so that frame - 2 of its first frames names no earlier record
+        if (ws->next_stamp + max_frames + 16 > 0xffffffffull) {
+            FF_CUDA_CHECK(cudaMemsetAsync(w.pend, 0, sizeof(SlotPend) * 2ull * P, stream));
+            ws->next_stamp = kFirstStamp;
+        }
+        w.stamp0 = (uint32_t)ws->next_stamp;
+        ws->next_stamp += (uint64_t)max_frames + 16;
+    }
     int shade_blocks = ctx->num_sms * 8;
     int n_kinds = 0;
     for (int k = 0; k < kKinds; ++k) n_kinds += kind_used[k] ? 1 : 0;
@@ -1068,7 +1085,6 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     uint32_t active = 1;
     ws->ensure_streams();
     uint32_t* h_active = ws->h_active();
-    const uint32_t max_frames = (st->spp + 1) * (st->max_depth + 2) + 8;
     // Deferred light terms (every render but the cached one): the any-hit
     // trace of frame f runs on the side stream beside k_logic, k_shade and
     // the closest-hit trace of frame f + 1, and k_logic of frame f + 2 adds
@@ -1080,6 +1096,7 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
         const uint32_t par = defer ? (f & 1u) : 0u;
         w.par = par;
         w.frame = f;
+        w.first = f == 0 ? 1u : 0u;
         w.ctr = ws->ctr_base + kCtrStride * par;
         w.sh_rays = ws->sh_rays_base[par];
         w.sh_tag = ws->sh_tag_base[par];
@@ -1194,8 +1211,8 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
         for (auto e : evs) cudaEventDestroy(e);
         // profiled renders add the two counting passes per frame
         // per frame: counter reset, logic, one shade per kind, two traces
-        // (+ two counting passes when profiled); init and resolve; the flush
-        stats->kernel_launches = frames * (4u + (uint32_t)n_kinds + (profile ? 2u : 0u)) + 2u + (defer ? 2u : 0u);
+        // (+ two counting passes when profiled); resolve; the flush
+        stats->kernel_launches = frames * (4u + (uint32_t)n_kinds + (profile ? 2u : 0u)) + 1u + (defer ? 2u : 0u);
         stats->extension_rays = ws->host_rays(0);
         stats->shadow_rays = ws->host_rays(1);
         stats->samples = (uint64_t)st->spp * WH;
@@ -1260,6 +1277,8 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     w.W = t.width;
     w.H = t.height;
     w.m = m;
+    w.spp = st->spp;
+    w.sample_offset = st->sample_offset;
     w.seed = st->seed;
     w.max_depth = st->max_depth;
     w.rr_depth = st->rr_depth;
@@ -1280,7 +1299,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     w.queries = nullptr;
     w.n_queries = nullptr;
     // no deferred light terms: the replay needs each vertex's answers at the next frame
-    w.defer = w.par = w.frame = 0u;
+    w.defer = w.par = w.frame = w.stamp0 = 0u;
     w.ctr = ws->ctr_base;
     w.sh_rays = ws->sh_rays_base[0];
     w.sh_tag = ws->sh_tag_base[0];
@@ -1304,8 +1323,6 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     int n_kinds = 0;
     for (int k = 0; k < kKinds; ++k) n_kinds += kind_used[k] ? 1 : 0;
 
-    k_init<<<(P + 255) / 256, 256, 0, stream>>>(w, st->spp, st->sample_offset);
-    FF_CUDA_CHECK(cudaGetLastError());
     const int shade_blocks = ctx->num_sms * 8;
     // optional per-stage timing, as in ff_wavefront_render
     const bool profile = stats && (st->flags & FF_RENDER_PROFILE);
@@ -1325,6 +1342,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     const uint32_t max_frames = 2 * (st->spp + 1) * (st->max_depth + 2) + 8;
     while (active && frames < max_frames) {
         for (int b = 0; b < 4; ++b) {
+            w.first = frames == 0 ? 1u : 0u;
             k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, ws->trace_ctr, w.totals);
             mark();
             k_logic<true><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
@@ -1378,7 +1396,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     }
     for (auto e : evs) cudaEventDestroy(e);
     if (stats) {
-        stats->kernel_launches = frames * (4u + (uint32_t)n_kinds) + 1u;   // counter reset, logic, shades, traces; init
+        stats->kernel_launches = frames * (4u + (uint32_t)n_kinds);   // counter reset, logic, shades, traces
         stats->extension_rays = ws->host_rays(0);
         stats->shadow_rays = ws->host_rays(1);
         stats->frames = frames;
