@@ -348,7 +348,7 @@ FF_API ff_status ff_render(ff_context* ctx, ff_scene* scene, const ff_render_set
 
 #define FF_ADJOINT_STORE_ALL 4u   /* ff_adjoint_desc.flags: store-all-vertices reference variant */
 #define FF_ADJOINT_MEGAKERNEL 16u /* ff_adjoint_desc.flags: one-thread-per-sample replay (cross-check) instead of
-                                     the wavefront replay */
+                                     the wavefront stages */
 #define FF_ENV_KEEP_TABLES   8u   /* ff_scene_set_environment: keep the importance tables */
 
 /* Gradient request of ff_render_adjoint.  d_image is dL/dI for the mean
@@ -370,14 +370,16 @@ typedef struct ff_adjoint_desc {
     float* grad_roughness;    /* NULL = no roughness gradient */
 } ff_adjoint_desc;
 
-/* Path-replay adjoint of ff_render (no counterpart in the reference, which
- * renders only): the same paths as ff_render in FF_MODE_CORRECTED for the same
- * settings (seed, spp, sample_offset, depths, light), replayed from their
- * seeds; gradients of the albedo texture of FF_MAT_DIFFUSE surfaces, of the
+/* Adjoint of ff_render (no counterpart in the reference, which renders
+ * only): the same paths as ff_render in FF_MODE_CORRECTED for the same
+ * settings (seed, spp, sample_offset, depths, light), their vertices kept until
+ * the sample's radiance is known, or, where that takes too much memory,
+ * replayed from their seeds; gradients of the albedo texture of FF_MAT_DIFFUSE surfaces, of the
  * roughness texture of GGX surfaces (FF_MAT_MIX, CONDUCTOR, DIELECTRIC, COAT)
  * and of the environment map (camera misses and NEE), with detached sampling
  * (directions, pdfs, MIS weights and the roulette are not differentiated).
- * settings->mode must be FF_MODE_CORRECTED.  stats: rays traced, samples,
+ * settings->mode must be FF_MODE_CORRECTED.  stats: the rays of the forward
+ * and the gradient pass (traced once where the vertices are kept), samples,
  * device time. */
 FF_API ff_status ff_render_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_settings* settings,
                                    const ff_adjoint_desc* desc, ff_render_stats* stats);
