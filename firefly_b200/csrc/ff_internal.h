@@ -175,6 +175,7 @@ struct ff_scene {
     DevBuf tangent;       // FFTangentTri[num_tris] when a material has a normal texture, else empty
     DevBuf materials;     // ff_material[num_materials]
     uint32_t num_materials = 0;
+    bool kind_used[FF_MAT_COAT + 1] = {};   // which ff_material_kind the materials have
     std::vector<DevBuf*> textures;
     DevBuf tex_table;     // device table of texture descriptors
     DevBuf area_lights;   // ff_area_light[]

@@ -154,6 +154,7 @@ void ff_build_shading(ff_context* ctx, ff_scene* s, const ff_scene_desc* d, cons
         s->tangent.release();
     }
     s->num_materials = (uint32_t)mats.size();
+    for (const ff_material& mt : mats) s->kind_used[mt.kind] = true;
     s->materials.alloc(sizeof(ff_material) * mats.size());
     FF_CUDA_CHECK(cudaMemcpyAsync(s->materials.ptr, mats.data(), sizeof(ff_material) * mats.size(),
                                   cudaMemcpyHostToDevice, st));

@@ -39,6 +39,8 @@
 // of that code.
 #include <algorithm>
 #include <cstddef>
+#include <cstring>
+#include <thread>
 #include <vector>
 
 #include "ff_adjoint.cuh"
@@ -62,13 +64,15 @@ constexpr uint32_t PH_FLIGHT = 1, PH_DONE = 2, PH_DRAINED = 3, kPhaseBits = 2;
 // fewer frames); 8M slots hold about 3.6 GB of path state.
 constexpr uint64_t kDefaultPoolTarget = 1ull << 23;
 
-// Counter words of one frame (zeroed at the start of each frame); one block
-// of kCtrStride words per frame parity.  C_EXT: extension rays of the frame,
+// Counter words of one frame, one block (an L2 line) for each of four
+// consecutive frames; k_logic of frame f clears the block of frame f + 2 (last
+// used by frame f - 2, whose traces are done then).  C_EXT: extension rays of the frame,
 // all of them counted by k_logic (its camera rays, C_CAM, and one
 // continuation per queued vertex); C_SH: shadow rays; C_MAT + k: vertices of
 // material kind k.
-enum { C_EXT = 0, C_SH = 1, C_MAT = 2, C_ACTIVE = 2 + kKinds, C_CAM = 3 + kKinds, C_WORDS = 8 + kKinds };
-constexpr uint32_t kCtrStride = 32;
+enum { C_EXT = 0, C_SH = 1, C_MAT = 2, C_ACTIVE = 2 + kKinds, C_CAM = 3 + kKinds,
+       C_TRACE = 16 /* 64-bit ray counters of the closest-hit and the any-hit trace */, C_WORDS = 20 };
+constexpr uint32_t kCtrStride = 32, kCtrRing = 4;
 
 // The slot's ray (origin, direction) and its visibility word: byte k = the
 // any-hit trace's answer for shadow ray k (1 occluded), byte 3 = which shadow
@@ -172,8 +176,11 @@ struct WF {
     ff_ray* sh_rays;
     uint32_t* sh_tag;    // per queued shadow ray: the byte of its answer (vis_byte, or 4 * slot + k in vis2)
     uint32_t* mat_queue;   // kKinds * P
-    uint32_t* ctr;         // C_WORDS
-    unsigned long long* totals;  // [0] extension rays, [1] shadow rays of the frames reset so far
+    uint32_t* ctr;         // the frame's counter block; ctr_next: that of frame + 2, ctr_last: that of frame - 1
+    uint32_t* ctr_next;
+    const uint32_t* ctr_last;
+    unsigned long long* totals;  // [0] extension rays, [1] shadow rays of the blocks cleared so far
+    volatile unsigned long long* progress;   // host memory, kProgress words: stamp0 + frame << 32 | active slots
     // scene
     const FFShadeTri* shade;
     const FFTangentTri* tan;   // tangent frames, or null when no material has a normal texture
@@ -221,6 +228,7 @@ struct WF {
     float4* rec2;
 };
 constexpr uint32_t kRecAlbedo = 2u;
+constexpr uint32_t kProgress = 64;
 // flags of WF::v_albedo.w: which gradients the vertex takes
 constexpr uint32_t V_ALBEDO = 1u, V_ROUGH = 2u, V_ENV = 4u, V_ROUGH_Y = 8u;   // V_ROUGH_Y: roughness in channel y
 
@@ -271,12 +279,12 @@ __device__ __forceinline__ void start_sample(const WF& w, uint32_t s, uint32_t s
 // their shadow rays' answers exactly as k_logic gates them without
 // deferral, into the slot's compensated sum.  Returns whether anything was
 // pending.
-__device__ __forceinline__ bool consume_pending(const WF& w, uint32_t s, float4& acc, float4& accc)
+__device__ __forceinline__ bool consume_pending(const WF& w, uint32_t frame, uint32_t s, float4& acc, float4& accc)
 {
-    const size_t i = (size_t)w.par * w.P + s;
+    const size_t i = (size_t)(frame & 1u) * w.P + s;
     const float4* pq = reinterpret_cast<const float4*>(w.pend + i);
     const float4 a = pq[0];
-    if (__float_as_uint(a.w) != w.stamp0 + w.frame - 2u) return false;
+    if (__float_as_uint(a.w) != w.stamp0 + frame - 2u) return false;
     const float4 b = pq[1];
     const uint32_t q = __float_as_uint(b.w);
     const uint32_t vw = w.vis2[i];
@@ -314,6 +322,22 @@ template <bool ADJ>
 __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0) {
+        // the counters of frame + 2 start from zero, after their last frame's
+        // rays join the totals; the host learns how many slots the last frame
+        // left active (with a launch of its own for the counters and a
+        // copy of the count that the host waited for every fourth frame, the 256
+        // x 256 preview took 639 us, so 501; 16 samples of it 2.24 and 2.15 ms, a
+        // 97 x 61 x 4 roughness adjoint 0.62 and 0.55 ms)
+        if (threadIdx.x < 2) w.totals[threadIdx.x] += w.ctr_next[threadIdx.x == 0 ? C_EXT : C_SH];
+        if (threadIdx.x == 2 && !w.first) {
+            w.progress[(w.frame - 1u) % kProgress] =
+                (unsigned long long)(w.stamp0 + w.frame - 1u) << 32 | w.ctr_last[C_ACTIVE];
+            __threadfence_system();
+        }
+        __syncwarp();
+        if (threadIdx.x < C_WORDS) w.ctr_next[threadIdx.x] = 0u;
+    }
     bool push_ext = false;   // the slot starts sample `sample`
     uint32_t sample = 0;
     int kind = -1;
@@ -347,7 +371,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
             float3 beta = xyz(beta4);
             float4 acc = w.acc[s];
             float4 accc = ADJ ? make_float4(0.f, 0.f, 0.f, 0.f) : w.acc_c[s];   // no compensation in the adjoint
-            if (!ADJ && w.defer) consume_pending(w, s, acc, accc);
+            if (!ADJ && w.defer) consume_pending(w, w.frame, s, acc, accc);
             bool terminate = (L > w.max_depth) || !found;
             // adjoint replay: dL/dI of this sample's pixel and the primal pass's L_s
             const bool record = ADJ && w.rec0;
@@ -588,7 +612,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
             // a slot that finished in the previous frame: the light terms of its
             // last vertex (shaded two frames ago) are the only ones still pending
             float4 acc = w.acc[s], accc = w.acc_c[s];
-            if (consume_pending(w, s, acc, accc)) {
+            if (consume_pending(w, w.frame, s, acc, accc)) {
                 w.acc[s] = acc;
                 w.acc_c[s] = accc;
             }
@@ -800,20 +824,9 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
     }
 }
 
-// Deferred mode: the light terms still pending after the last frame (stamp
-// w.frame - 2 of the parity of w.frame).
-__global__ void k_flush_pending(WF w)
-{
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= w.P) return;
-    float4 acc = w.acc[s], accc = w.acc_c[s];
-    if (consume_pending(w, s, acc, accc)) {
-        w.acc[s] = acc;
-        w.acc_c[s] = accc;
-    }
-}
-
 // Film += the m slot sums of each pixel, in slot order (compensated).
+// Deferred mode: w.frame is the number of frames run; the light terms still
+// pending after the last two join the sums first.
 __global__ void k_resolve(WF w, float4* __restrict__ film_acc, float4* __restrict__ film_c, uint32_t* __restrict__ film_n)
 {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -821,7 +834,11 @@ __global__ void k_resolve(WF w, float4* __restrict__ film_acc, float4* __restric
     float4 sum = film_acc[p], c = film_c[p];
     for (uint32_t k = 0; k < w.m; ++k) {
         const uint32_t s = p + k * w.WH;
-        const float4 a = w.acc[s], ac = w.acc_c[s];
+        float4 a = w.acc[s], ac = w.acc_c[s];
+        if (w.defer) {
+            consume_pending(w, w.frame, s, a, ac);
+            consume_pending(w, w.frame + 1u, s, a, ac);
+        }
         kahan_add(sum, c, make_float3(a.x - ac.x, a.y - ac.y, a.z - ac.z));
     }
     film_acc[p] = sum;
@@ -829,23 +846,11 @@ __global__ void k_resolve(WF w, float4* __restrict__ film_acc, float4* __restric
     film_n[p] += w.spp;
 }
 
-// Adds the rays of the last frame that used these counters to the totals
-// (extension, shadow) and clears the counters for the next one.
-__global__ void k_reset_counters(uint32_t* ctr, unsigned long long* trace_counters, unsigned long long* totals)
-{
-    if (threadIdx.x < 2) {
-        totals[threadIdx.x] += ctr[threadIdx.x == 0 ? C_EXT : C_SH];
-        trace_counters[threadIdx.x] = 0ull;
-    }
-    __syncthreads();
-    if (threadIdx.x < C_WORDS) ctr[threadIdx.x] = 0;
-}
-
 }  // namespace
 
 // Byte offsets of the control block's parts (each carved to a 256-byte boundary).
-constexpr size_t kCtlTotals = 256, kCtlErr = 512, kCtlFetch = 1024, kCtlBytes = 1280;
-static_assert(2 * kCtrStride * sizeof(uint32_t) == kCtlTotals, "two parities' counter words fill the first part");
+constexpr size_t kCtlTotals = 512, kCtlErr = 768, kCtlFetch = 1024, kCtlBytes = 1280;
+static_assert(kCtrRing * kCtrStride * sizeof(uint32_t) == kCtlTotals, "the counter blocks fill the first part");
 
 // Per-film workspace: slot arrays and queues, reused while the pool size is unchanged.
 struct FFWavefrontWS {
@@ -859,33 +864,40 @@ struct FFWavefrontWS {
     uint32_t adj_P = 0;
     WF w{};
     unsigned int* err = nullptr;
-    unsigned long long* trace_ctr = nullptr;  // per frame parity p: [2p] closest, [2p + 1] any
-    // per frame parity p: the counter words (ctr_base + kCtrStride * p) and the
-    // shadow queue (sh_rays_base[p], sh_tag_base[p]); WF points at the current
-    // frame's
+    // the counter blocks (frame f's at ctr_base + kCtrStride * (f % kCtrRing))
+    // and per frame parity p the shadow queue (sh_rays_base[p],
+    // sh_tag_base[p]); WF points at the current frame's
     uint32_t* ctr_base = nullptr;
     ff_ray* sh_rays_base[2] = {nullptr, nullptr};
     uint32_t* sh_tag_base[2] = {nullptr, nullptr};
     unsigned long long* fetch = nullptr;      // profiled renders: nodes / tris of the closest, then the any-hit traces
-    // the counter words, totals, error count, trace counters and fetch counts
-    // are carved one after the other (kCtlBytes from ctr_base): one memset
-    // clears them, one copy brings them to this pinned block
+    // the counter blocks, totals, error count and fetch counts are carved one
+    // after the other (kCtlBytes from ctr_base): one memset clears them, one
+    // copy brings them to this pinned block, which WF::progress follows
     char* h_ctl = nullptr;
+    volatile unsigned long long* progress() const
+    {
+        return reinterpret_cast<volatile unsigned long long*>(h_ctl + kCtlBytes);
+    }
     // extension ([0]) and shadow ([1]) rays of the call, from h_ctl: the
-    // totals of the frames reset so far and the counters of the last ones
+    // totals of the blocks cleared so far and the counters of the last frames
     uint64_t host_rays(int k) const
     {
         const uint32_t* c = reinterpret_cast<const uint32_t*>(h_ctl);
         const uint64_t* t = reinterpret_cast<const uint64_t*>(h_ctl + kCtlTotals);
-        const int word = k == 0 ? C_EXT : C_SH;
-        return t[k] + c[word] + c[kCtrStride + word];
+        uint64_t n = t[k];
+        for (uint32_t b = 0; b < kCtrRing; ++b) n += c[b * kCtrStride + (k == 0 ? C_EXT : C_SH)];
+        return n;
+    }
+    uint32_t host_active(uint32_t frame) const
+    {
+        return reinterpret_cast<const uint32_t*>(h_ctl)[(frame % kCtrRing) * kCtrStride + C_ACTIVE];
     }
     unsigned int host_err() const { return *reinterpret_cast<const unsigned int*>(h_ctl + kCtlErr); }
     const unsigned long long* host_fetch() const
     {
         return reinterpret_cast<const unsigned long long*>(h_ctl + kCtlFetch);
     }
-    uint32_t* h_active() const { return reinterpret_cast<uint32_t*>(h_ctl); }
     // the any-hit trace runs on `side` beside the closest-hit trace: its
     // blocks take the SMs the closest-hit trace's finished blocks leave
     cudaStream_t side = nullptr;
@@ -983,7 +995,7 @@ size_t ws_bytes(uint32_t P)
     add(16, P) /*beta*/; add(sizeof(SlotRay), P); add(sizeof(SlotShade), P); add(sizeof(SlotMis), P);
     add(sizeof(SlotVtx), P); add(16, P) /*hit_ngeo*/; add(16, P); add(16, P) /*acc, acc_c*/;
     add(sizeof(ff_ray), P); add(4, P); add(sizeof(ff_hit), P); add(sizeof(ff_ray), 3ull * P); add(4, 3ull * P);
-    add(4, (size_t)kKinds * P); add(4, 2 * kCtrStride); add(8, 8); add(4, 4); add(8, 4); add(8, 4);
+    add(4, (size_t)kKinds * P); add(4, kCtrRing * kCtrStride); add(8, 8); add(4, 4); add(8, 4);
     return b;
 }
 
@@ -1013,13 +1025,16 @@ void ws_setup(FFWavefrontWS* ws, uint32_t P)
     ws->sh_rays_base[0] = w.sh_rays = carve<ff_ray>(p, 3ull * P);
     ws->sh_tag_base[0] = w.sh_tag = carve<uint32_t>(p, 3ull * P);
     w.mat_queue = carve<uint32_t>(p, (size_t)kKinds * P);
-    ws->ctr_base = w.ctr = carve<uint32_t>(p, 2 * kCtrStride);
+    ws->ctr_base = w.ctr = carve<uint32_t>(p, kCtrRing * kCtrStride);
     w.defer = w.par = w.frame = w.first = 0u;
     w.totals = carve<unsigned long long>(p, 8);
     ws->err = carve<unsigned int>(p, 4);
-    ws->trace_ctr = carve<unsigned long long>(p, 4);
     ws->fetch = carve<unsigned long long>(p, 4);
-    if (!ws->h_ctl) FF_CUDA_CHECK(cudaMallocHost(&ws->h_ctl, kCtlBytes));
+    if (!ws->h_ctl) {
+        constexpr size_t bytes = kCtlBytes + kProgress * sizeof(unsigned long long);
+        FF_CUDA_CHECK(cudaMallocHost(&ws->h_ctl, bytes));
+        std::memset(ws->h_ctl, 0, bytes);   // no frame's report: stamps start at kFirstStamp
+    }
     ws->sh_rays_base[1] = nullptr;
     ws->sh_tag_base[1] = nullptr;
     w.pend = nullptr;
@@ -1047,9 +1062,79 @@ void defer_setup(FFWavefrontWS* ws, uint32_t P, cudaStream_t stream)
     ws->w.pend = carve<SlotPend>(p, 2ull * P);
     ws->w.vis2 = carve<uint32_t>(p, 2ull * P);
     FF_CUDA_CHECK(cudaMemsetAsync(ws->w.pend, 0, sizeof(SlotPend) * 2ull * P, stream));
-    ws->next_stamp = kFirstStamp;
     ws->defer_P = P;
 }
+
+// The frames of one render: counter blocks, stamps, and how far the host may
+// run ahead.
+struct FrameLoop {
+    FFWavefrontWS* ws;
+    cudaStream_t stream;
+    uint32_t frames = 0;   // launched
+    uint32_t cap;          // frames that always suffice
+    // `passes` passes over each sample; a sample takes at most max_depth + 1
+    // frames a pass, the next one starts in the frame that ends it, and frame
+    // 0 starts the first
+    FrameLoop(FFWavefrontWS* ws_, cudaStream_t stream_, const WF& w, uint32_t passes) : ws(ws_), stream(stream_)
+    {
+        const uint64_t per_slot = (w.spp + w.m - 1) / w.m;
+        const uint64_t need = passes * per_slot * (w.max_depth + 1) + 1;
+        FF_REQUIRE(need < (1ull << 31), "too many frames in one call");
+        cap = (uint32_t)need;
+        // stamps of frames 0, 1, ... of this render: above those of the renders
+        // before it, with room for the frame - 2 of its first frames and the
+        // frame + 1 of its last
+        if (ws->next_stamp + need + 16 > 0xffffffffull) {
+            if (ws->w.pend)
+                FF_CUDA_CHECK(cudaMemsetAsync(ws->w.pend, 0, sizeof(SlotPend) * 2ull * ws->P, stream));
+            for (uint32_t k = 0; k < kProgress; ++k) ws->progress()[k] = 0;
+            ws->next_stamp = kFirstStamp;
+        }
+        ws->w.stamp0 = (uint32_t)ws->next_stamp;
+        ws->next_stamp += need + 16;
+        ws->w.progress = ws->progress();
+        FF_CUDA_CHECK(cudaMemsetAsync(ws->ctr_base, 0, kCtlBytes, stream));
+    }
+    // Points WF at the next frame; false when no frame is left to run.  The
+    // host waits for the active count that k_logic of the frame before the
+    // last one's successor reports, so one frame is always queued behind the
+    // running one and at most one empty frame runs at the end.
+    bool next(WF& w)
+    {
+        if (frames >= cap || (frames >= 2 && active_after(frames - 2) == 0)) return false;
+        w.frame = frames;
+        w.first = frames == 0 ? 1u : 0u;
+        w.ctr = ws->ctr_base + kCtrStride * (frames % kCtrRing);
+        w.ctr_next = ws->ctr_base + kCtrStride * ((frames + 2) % kCtrRing);
+        w.ctr_last = ws->ctr_base + kCtrStride * ((frames + kCtrRing - 1) % kCtrRing);
+        ++frames;
+        return true;
+    }
+    // whether the frame next() pointed at can have vertices (frame 0 only
+    // starts paths) and rays (every path has ended in the last possible one)
+    bool has_vertices() const { return frames > 1 && has_rays(); }
+    bool has_rays() const { return frames < cap; }
+    // Slots active after frame f, reported by k_logic of frame f + 1 (launched).
+    uint32_t active_after(uint32_t f)
+    {
+        const unsigned long long stamp = (unsigned long long)ws->w.stamp0 + f;
+        volatile unsigned long long* p = ws->progress() + f % kProgress;
+        for (uint32_t spin = 1;; ++spin) {
+            unsigned long long v = *p;
+            if (v >> 32 == stamp) return (uint32_t)v;
+            if (spin % 4096u == 0u) {
+                const cudaError_t e = cudaStreamQuery(stream);
+                if (e == cudaSuccess) {
+                    v = *p;
+                    if (v >> 32 == stamp) return (uint32_t)v;
+                    throw FFError{FF_ERR_INTERNAL, "wavefront frame left no progress report"};
+                }
+                if (e != cudaErrorNotReady) FF_CUDA_CHECK(e);
+                std::this_thread::yield();
+            }
+        }
+    }
+};
 
 }  // namespace
 
@@ -1103,31 +1188,12 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     }
     const FFBvhView bvh = scene->view();
 
-    // which material kinds occur
-    std::vector<ff_material> mats(scene->num_materials);
-    FF_CUDA_CHECK(cudaMemcpyAsync(mats.data(), scene->materials.ptr, sizeof(ff_material) * mats.size(),
-                                  cudaMemcpyDeviceToHost, stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(ws->ctr_base, 0, kCtlBytes, stream));
-    FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-    bool kind_used[kKinds] = {false, false, false, false, false};
-    for (auto& mt : mats) kind_used[mt.kind] = true;
-
+    const bool* kind_used = scene->kind_used;
     // deferred light terms: every render but the cached one (see the frame loop)
     const bool defer = hook == nullptr;
     w.defer = defer ? 1u : 0u;
-    const uint32_t max_frames = (st->spp + 1) * (st->max_depth + 2) + 8;
     FF_CUDA_CHECK(cudaEventRecord(ctx->ev0, stream));
-    if (defer) {
-        defer_setup(ws, P, stream);
-        // stamps of frames 0, 1, ... of this render, two above the last one's
-        // so that frame - 2 of its first frames names no earlier record
-        if (ws->next_stamp + max_frames + 16 > 0xffffffffull) {
-            FF_CUDA_CHECK(cudaMemsetAsync(w.pend, 0, sizeof(SlotPend) * 2ull * P, stream));
-            ws->next_stamp = kFirstStamp;
-        }
-        w.stamp0 = (uint32_t)ws->next_stamp;
-        ws->next_stamp += (uint64_t)max_frames + 16;
-    }
+    if (defer) defer_setup(ws, P, stream);
     int shade_blocks = ctx->num_sms * 8;
     int n_kinds = 0;
     for (int k = 0; k < kKinds; ++k) n_kinds += kind_used[k] ? 1 : 0;
@@ -1141,38 +1207,29 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
         FF_CUDA_CHECK(cudaEventRecord(e, stream));
         evs.push_back(e);
     };
-    uint32_t frames = 0;
-    uint32_t active = 1;
     ws->ensure_streams();
-    uint32_t* h_active = ws->h_active();
+    FrameLoop loop(ws, stream, w, 1);
+    uint32_t launches = 1;   // k_resolve
     // Deferred light terms (every render but the cached one): the any-hit
     // trace of frame f runs on the side stream beside k_logic, k_shade and
     // the closest-hit trace of frame f + 1, and k_logic of frame f + 2 adds
-    // the light terms its answers let through.  Frames of one parity share
-    // counters, a shadow queue and pending records, so frame f + 2 waits for
-    // the any-hit trace of frame f.  Under stage timing everything stays on
-    // the one stream.
-    auto set_frame = [&](uint32_t f) -> uint32_t {
-        const uint32_t par = defer ? (f & 1u) : 0u;
+    // the light terms its answers let through.  Frames of one parity share a
+    // shadow queue and pending records, so frame f + 2 waits for the any-hit
+    // trace of frame f.  Under stage timing everything stays on the one
+    // stream.
+    while (loop.next(w)) {
+        const uint32_t par = defer ? (w.frame & 1u) : 0u;
         w.par = par;
-        w.frame = f;
-        w.first = f == 0 ? 1u : 0u;
-        w.ctr = ws->ctr_base + kCtrStride * par;
         w.sh_rays = ws->sh_rays_base[par];
         w.sh_tag = ws->sh_tag_base[par];
-        return par;
-    };
-    while (active && frames < max_frames) {
-        // a batch of frames between host checks
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t par = set_frame(frames);
-            unsigned long long* tctr = ws->trace_ctr + 2 * par;
-            uint8_t* occ = defer ? reinterpret_cast<uint8_t*>(w.vis2 + (size_t)par * P) : reinterpret_cast<uint8_t*>(w.ray);
-            if (defer && !profile && frames >= 2) FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[par], 0));
-            k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, tctr, w.totals);
-            mark();
-            k_logic<false><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
-            mark();
+        unsigned long long* tctr = reinterpret_cast<unsigned long long*>(w.ctr + C_TRACE);
+        uint8_t* occ = defer ? reinterpret_cast<uint8_t*>(w.vis2 + (size_t)par * P) : reinterpret_cast<uint8_t*>(w.ray);
+        if (defer && !profile && w.frame >= 2) FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[par], 0));
+        mark();
+        k_logic<false><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
+        ++launches;
+        mark();
+        if (loop.has_vertices()) {
             // with stage timing (profile) every launch stays on the one stream
             FFWavefrontWS* side = profile ? nullptr : ws;
             const bool sel = w.lights.light == FF_LIGHT_ALL, corr = w.mode == FF_MODE_CORRECTED;
@@ -1180,55 +1237,51 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
             if (sel) launch_shade<true, false, true>(w, kind_used, shade_blocks, stream, side);
             else if (corr) launch_shade<false, false, true>(w, kind_used, shade_blocks, stream, side);
             else launch_shade<false, false, false>(w, kind_used, shade_blocks, stream, side);
-            FF_CUDA_CHECK(cudaGetLastError());
-            mark();
-            if (profile) {
-                // stage timing: the two traces one after the other
-                ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, tctr, ws->err,
-                                      w.ext_tag, nullptr, nullptr, scene->refracts);
-                mark();
-                ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true, tctr + 1, ws->err,
-                                      w.sh_tag, occ);
-                mark();
-                // the traversal work of this frame's queues, counted by a second pass of the same
-                // traversal (outside the stage marks)
-                ff_launch_trace_count_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, false, scene->refracts, ws->fetch,
-                                            ws->err, stream);
-                ff_launch_trace_count_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, true, false, ws->fetch + 2,
-                                            ws->err, stream);
-            } else {
-                // the traces are independent (hits by slot, answers by shadow-ray tag)
-                FF_CUDA_CHECK(cudaEventRecord(ws->fork, stream));
-                FF_CUDA_CHECK(cudaStreamWaitEvent(ws->side, ws->fork, 0));
-                ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, tctr, ws->err,
-                                      w.ext_tag, nullptr, nullptr, scene->refracts);
-                ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true, tctr + 1, ws->err,
-                                      w.sh_tag, occ, ws->side, false, defer ? kDeferShadowBlocks : 0);
-                if (defer) {
-                    FF_CUDA_CHECK(cudaEventRecord(ws->sh_done[par], ws->side));
-                } else {
-                    FF_CUDA_CHECK(cudaEventRecord(ws->join, ws->side));
-                    FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->join, 0));
-                }
-            }
-            ++frames;
-        }
-        FF_CUDA_CHECK(cudaMemcpyAsync(h_active, w.ctr + C_ACTIVE, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-        active = *h_active;
-    }
-    if (active) throw FFError{FF_ERR_INTERNAL, "wavefront did not finish within its frame bound"};
-    if (defer) {
-        // the light terms of the last two frames, once their any-hit traces are done
-        if (!profile) {
-            FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[0], 0));
-            FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[1], 0));
-        }
-        for (uint32_t f = frames; f < frames + 2; ++f) {
-            set_frame(f);
-            k_flush_pending<<<(P + 255) / 256, 256, 0, stream>>>(w);
+            launches += (uint32_t)n_kinds;
         }
         FF_CUDA_CHECK(cudaGetLastError());
+        mark();
+        // the traces are independent (hits by slot, answers by shadow-ray tag)
+        const bool fork = loop.has_vertices() && !profile;
+        if (fork) {
+            FF_CUDA_CHECK(cudaEventRecord(ws->fork, stream));
+            FF_CUDA_CHECK(cudaStreamWaitEvent(ws->side, ws->fork, 0));
+        }
+        if (loop.has_rays()) {
+            ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, tctr, ws->err,
+                                  w.ext_tag, nullptr, nullptr, scene->refracts);
+            ++launches;
+        }
+        mark();
+        if (loop.has_vertices()) {
+            ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true, tctr + 1, ws->err,
+                                  w.sh_tag, occ, fork ? ws->side : nullptr, false,
+                                  fork && defer ? kDeferShadowBlocks : 0);
+            ++launches;
+        }
+        mark();
+        if (fork && defer) {
+            FF_CUDA_CHECK(cudaEventRecord(ws->sh_done[par], ws->side));
+        } else if (fork) {
+            FF_CUDA_CHECK(cudaEventRecord(ws->join, ws->side));
+            FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->join, 0));
+        }
+        if (profile && loop.has_rays()) {
+            // the traversal work of this frame's queues, counted by a second pass of the same
+            // traversal (outside the stage marks)
+            ff_launch_trace_count_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, false, scene->refracts, ws->fetch,
+                                        ws->err, stream);
+            ff_launch_trace_count_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, true, false, ws->fetch + 2,
+                                        ws->err, stream);
+            launches += 2;
+        }
+    }
+    const uint32_t frames = loop.frames;
+    w.frame = frames;
+    if (defer && !profile) {
+        // the light terms of the last two frames wait for their any-hit traces
+        FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[0], 0));
+        FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[1], 0));
     }
     // cache answers join their slots' sums before the film update
     if (hook) {
@@ -1244,6 +1297,7 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     FF_CUDA_CHECK(cudaMemcpyAsync(ws->h_ctl, ws->ctr_base, kCtlBytes, cudaMemcpyDeviceToHost, stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(stream));
     const unsigned long long* fetch = ws->host_fetch();
+    if (ws->host_active(frames - 1)) throw FFError{FF_ERR_INTERNAL, "wavefront did not finish within its frame bound"};
     if (ws->host_err()) throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
     if (stats) {
         float ms = 0.f;
@@ -1269,10 +1323,7 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
             stats->ms_trace_shadow = t[3];
         }
         for (auto e : evs) cudaEventDestroy(e);
-        // profiled renders add the two counting passes per frame
-        // per frame: counter reset, logic, one shade per kind, two traces
-        // (+ two counting passes when profiled); resolve; the flush
-        stats->kernel_launches = frames * (4u + (uint32_t)n_kinds + (profile ? 2u : 0u)) + 1u + (defer ? 2u : 0u);
+        stats->kernel_launches = launches;   // (the caller counts the cache's inference)
         stats->extension_rays = ws->host_rays(0);
         stats->shadow_rays = ws->host_rays(1);
         stats->samples = (uint64_t)st->spp * WH;
@@ -1389,8 +1440,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     w.queries = nullptr;
     w.n_queries = nullptr;
     // no deferred light terms: the replay needs each vertex's answers at the next frame
-    w.defer = w.par = w.frame = w.stamp0 = 0u;
-    w.ctr = ws->ctr_base;
+    w.defer = w.par = 0u;
     w.sh_rays = ws->sh_rays_base[0];
     w.sh_tag = ws->sh_tag_base[0];
     w.d_image = t.d_image;
@@ -1403,13 +1453,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     w.touched = t.touched;
     const FFBvhView bvh = scene->view();
 
-    std::vector<ff_material> mats(scene->num_materials);
-    FF_CUDA_CHECK(cudaMemcpyAsync(mats.data(), scene->materials.ptr, sizeof(ff_material) * mats.size(),
-                                  cudaMemcpyDeviceToHost, stream));
-    FF_CUDA_CHECK(cudaMemsetAsync(ws->ctr_base, 0, kCtlBytes, stream));
-    FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-    bool kind_used[kKinds] = {false, false, false, false, false};
-    for (auto& mt : mats) kind_used[mt.kind] = true;
+    const bool* kind_used = scene->kind_used;
     int n_kinds = 0;
     for (int k = 0; k < kKinds; ++k) n_kinds += kind_used[k] ? 1 : 0;
 
@@ -1424,50 +1468,49 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
         FF_CUDA_CHECK(cudaEventRecord(e, stream));
         evs.push_back(e);
     };
-    uint32_t frames = 0;
-    uint32_t active = 1;
     ws->ensure_streams();
-    uint32_t* h_active = ws->h_active();
-    // two passes per sample
-    const uint32_t max_frames = 2 * (st->spp + 1) * (st->max_depth + 2) + 8;
-    while (active && frames < max_frames) {
-        for (int b = 0; b < 4; ++b) {
-            w.first = frames == 0 ? 1u : 0u;
-            k_reset_counters<<<1, 32, 0, stream>>>(w.ctr, ws->trace_ctr, w.totals);
-            mark();
-            k_logic<true><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
-            mark();
-            // side streams as in ff_wavefront_render (one stream under stage timing)
+    FrameLoop loop(ws, stream, w, w.rec0 ? 1 : 2);
+    uint32_t launches = 0;
+    while (loop.next(w)) {
+        unsigned long long* tctr = reinterpret_cast<unsigned long long*>(w.ctr + C_TRACE);
+        mark();
+        k_logic<true><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
+        ++launches;
+        mark();
+        // side streams as in ff_wavefront_render (one stream under stage timing)
+        if (loop.has_vertices()) {
             launch_shade<false, true, true>(w, kind_used, shade_blocks, stream, profile ? nullptr : ws);
-            FF_CUDA_CHECK(cudaGetLastError());
-            mark();
-            if (profile) {
-                ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, ws->trace_ctr,
-                                      ws->err, w.ext_tag, nullptr, nullptr, scene->refracts);
-                mark();
-                ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true,
-                                      ws->trace_ctr + 1, ws->err, w.sh_tag, reinterpret_cast<uint8_t*>(w.ray));
-                mark();
-            } else {
-                FF_CUDA_CHECK(cudaEventRecord(ws->fork, stream));
-                FF_CUDA_CHECK(cudaStreamWaitEvent(ws->side, ws->fork, 0));
-                ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, ws->trace_ctr,
-                                      ws->err, w.ext_tag, nullptr, nullptr, scene->refracts);
-                ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true,
-                                      ws->trace_ctr + 1, ws->err, w.sh_tag, reinterpret_cast<uint8_t*>(w.ray),
-                                      ws->side);
-                FF_CUDA_CHECK(cudaEventRecord(ws->join, ws->side));
-                FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->join, 0));
-            }
-            ++frames;
+            launches += (uint32_t)n_kinds;
         }
-        FF_CUDA_CHECK(cudaMemcpyAsync(h_active, w.ctr + C_ACTIVE, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-        FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-        active = *h_active;
+        FF_CUDA_CHECK(cudaGetLastError());
+        mark();
+        const bool fork = loop.has_vertices() && !profile;
+        if (fork) {
+            FF_CUDA_CHECK(cudaEventRecord(ws->fork, stream));
+            FF_CUDA_CHECK(cudaStreamWaitEvent(ws->side, ws->fork, 0));
+        }
+        if (loop.has_rays()) {
+            ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, tctr, ws->err, w.ext_tag,
+                                  nullptr, nullptr, scene->refracts);
+            ++launches;
+        }
+        mark();
+        if (loop.has_vertices()) {
+            ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true, tctr + 1, ws->err,
+                                  w.sh_tag, reinterpret_cast<uint8_t*>(w.ray), fork ? ws->side : nullptr);
+            ++launches;
+        }
+        mark();
+        if (fork) {
+            FF_CUDA_CHECK(cudaEventRecord(ws->join, ws->side));
+            FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->join, 0));
+        }
     }
-    if (active) throw FFError{FF_ERR_INTERNAL, "wavefront adjoint did not finish within its frame bound"};
+    const uint32_t frames = loop.frames;
     FF_CUDA_CHECK(cudaMemcpyAsync(ws->h_ctl, ws->ctr_base, kCtlBytes, cudaMemcpyDeviceToHost, stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(stream));
+    if (ws->host_active(frames - 1))
+        throw FFError{FF_ERR_INTERNAL, "wavefront adjoint did not finish within its frame bound"};
     if (ws->host_err()) throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
     if (profile) {
         // 5 marks per frame: logic | shade | trace extension | trace shadow
@@ -1486,7 +1529,7 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     }
     for (auto e : evs) cudaEventDestroy(e);
     if (stats) {
-        stats->kernel_launches = frames * (4u + (uint32_t)n_kinds);   // counter reset, logic, shades, traces
+        stats->kernel_launches = launches;
         // the rays of both passes over each path; with records the second
         // pass takes its answers from them
         const uint64_t passes = w.rec0 ? 2u : 1u;
