@@ -106,9 +106,9 @@ struct ff_context {
     DevBuf adj_io[5];         // ff_render_adjoint: staged image, texture / env / roughness gradients, counters
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     FFWavefrontWS* adj_ws = nullptr;   // path pool of ff_render_adjoint, kept between calls
-    // resident blocks per SM of each queue-driven k_trace variant on this
-    // context's device (0 = not yet queried), indexed by any-hit | tagged << 1 | two-sided << 2
-    int trace_bps[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // resident blocks per SM of each trace kernel on this context's device (0 =
+    // not yet queried), indexed by any-hit | tagged << 1 | two-sided << 2 | eight lanes a ray << 3
+    int trace_bps[16] = {};
 };
 
 // Per-original-triangle shading attributes, read once per hit by a gather

@@ -165,8 +165,17 @@ FF_D void ff_intersect_node(const FFNode8* __restrict__ nodes, uint32_t idx, con
 // some lane nearly always reaches the last FP32 comparison, so leaving at
 // each one only adds branches (3M any-hit rays on the 1.3M-triangle mesh 241
 // -> 230 us, its 64-spp step 240.4 -> 234.8 ms).
-template <bool TWO = false>
-FF_D void ff_test_tri_closest(const FFTri* __restrict__ tris, uint32_t k, FFRayState& r)
+struct FFCandidate {
+    float t, uf, vf;   // uf, vf: numerators of u and v over det
+    double inv_det;
+    uint32_t id;       // original index
+    bool back;         // a back face (TWO)
+    FF_D float u() const { return __double2float_rn(__dmul_rn((double)uf, inv_det)); }
+    FF_D float v() const { return __double2float_rn(__dmul_rn((double)vf, inv_det)); }
+};
+// The test but for the comparison with the best hit so far.
+template <bool TWO>
+FF_D bool ff_candidate(const FFTri* __restrict__ tris, uint32_t k, const FFRayState& r, FFCandidate& h)
 {
     const float4 a = __ldg(&tris[k].a);
     const float4 b = __ldg(&tris[k].b);
@@ -179,37 +188,50 @@ FF_D void ff_test_tri_closest(const FFTri* __restrict__ tris, uint32_t k, FFRayS
     bool out = det < FF_K_EPSILON;
     float sg = 1.f;
     if (TWO) {
-        const bool back = signbit(r.tmin) && det <= -FF_K_EPSILON;
-        sg = back ? -1.f : 1.f;
-        det = back ? -det : det;
-        out = out && !back;
+        h.back = signbit(r.tmin) && det <= -FF_K_EPSILON;
+        sg = h.back ? -1.f : 1.f;
+        det = h.back ? -det : det;
+        out = out && !h.back;
     }
     const float3 tvec = rn_sub(r.o, v0);
-    const float uf = TWO ? sg * rn_dot(tvec, pvec) : rn_dot(tvec, pvec);
-    out |= (uf < 0.f) | (uf > det);
+    h.uf = TWO ? sg * rn_dot(tvec, pvec) : rn_dot(tvec, pvec);
+    out |= (h.uf < 0.f) | (h.uf > det);
     const float3 qvec = rn_cross(tvec, e1);
-    const float vf = TWO ? sg * rn_dot(r.d, qvec) : rn_dot(r.d, qvec);
-    out |= (vf < 0.f) | (__fadd_rn(uf, vf) > det);
+    h.vf = TWO ? sg * rn_dot(r.d, qvec) : rn_dot(r.d, qvec);
+    out |= (h.vf < 0.f) | (__fadd_rn(h.uf, h.vf) > det);
     const float tf = TWO ? sg * rn_dot(e2, qvec) : rn_dot(e2, qvec);
-    if (out) return;
-    const double inv_det = __drcp_rn((double)det);
-    const float t = __double2float_rn(__dmul_rn((double)tf, inv_det));
-    if (t < 0.f || !(t >= (TWO ? fabsf(r.tmin) : r.tmin))) return;
-    const uint32_t id = (uint32_t)__float_as_int(a.w);
+    if (out) return false;
+    h.inv_det = __drcp_rn((double)det);
+    h.t = __double2float_rn(__dmul_rn((double)tf, h.inv_det));
+    h.id = (uint32_t)__float_as_int(a.w);
+    return !(h.t < 0.f) && h.t >= (TWO ? fabsf(r.tmin) : r.tmin);
+}
+// Whether a candidate replaces the best hit so far.
+template <bool TWO>
+FF_D bool ff_better(const FFRayState& r, float t, uint32_t id)
+{
     const uint32_t best = TWO ? (r.prim & ~kBackFace) : r.prim;
-    if (t < r.tmax || (t == r.tmax && r.prim != 0xffffffffu && id < best)) {
-        r.tmax = t;
-        r.prim = (TWO && sg < 0.f) ? (id | kBackFace) : id;
-        r.u = __double2float_rn(__dmul_rn((double)uf, inv_det));
-        r.v = __double2float_rn(__dmul_rn((double)vf, inv_det));
+    return t < r.tmax || (t == r.tmax && r.prim != 0xffffffffu && id < best);
+}
+
+template <bool TWO = false>
+FF_D void ff_test_tri_closest(const FFTri* __restrict__ tris, uint32_t k, FFRayState& r)
+{
+    FFCandidate h;
+    if (ff_candidate<TWO>(tris, k, r, h) && ff_better<TWO>(r, h.t, h.id)) {
+        r.tmax = h.t;
+        r.prim = (TWO && h.back) ? (h.id | kBackFace) : h.id;
+        r.u = h.u();
+        r.v = h.v();
     }
 }
 
 // dTriangle::shadow_hit (CUDA-RayTracer/dTriangle.cu:110-138) and the
-// t < tmin test of intersect_shadows (:233).  Returns true on an occluder.
-// An FP32 pre-test rejects candidates that the FP64 test would certainly
-// reject (sign of u, v and u + v > 1 with margin); the FP64 test decides the rest.
-FF_D bool ff_test_tri_any(const FFTri* __restrict__ tris, uint32_t k, FFRayState& r)
+// t < tmin test of intersect_shadows (:233).  Returns true on an occluder,
+// with its t and original index.  An FP32 pre-test rejects candidates that
+// the FP64 test would certainly reject (sign of u, v and u + v > 1 with
+// margin); the FP64 test decides the rest.
+FF_D bool ff_occluder(const FFTri* __restrict__ tris, uint32_t k, const FFRayState& r, float& t, uint32_t& id)
 {
     const float4 a = __ldg(&tris[k].a);
     const float4 b = __ldg(&tris[k].b);
@@ -235,14 +257,19 @@ FF_D bool ff_test_tri_any(const FFTri* __restrict__ tris, uint32_t k, FFRayState
     const double v = __dmul_rn((double)vf, inv_det);
     if (v < 0.0 || __dadd_rn(u, v) > 1.0) return false;
     const float tf = rn_dot(e2, qvec);
-    const float t = __double2float_rn(__dmul_rn((double)tf, inv_det));
-    if (t < 0.f) return false;
-    if (t >= r.tmin && t < r.tmax) {
-        r.prim = (uint32_t)__float_as_int(a.w);
-        r.tmax = t;  // the traversal ends here; tmax now reports the occluder's t
-        return true;
-    }
-    return false;
+    t = __double2float_rn(__dmul_rn((double)tf, inv_det));
+    id = (uint32_t)__float_as_int(a.w);
+    return !(t < 0.f) && t >= r.tmin && t < r.tmax;
+}
+
+FF_D bool ff_test_tri_any(const FFTri* __restrict__ tris, uint32_t k, FFRayState& r)
+{
+    float t;
+    uint32_t id;
+    if (!ff_occluder(tris, k, r, t, id)) return false;
+    r.prim = id;
+    r.tmax = t;  // the traversal ends here; tmax now reports the occluder's t
+    return true;
 }
 
 // Traversal stack: kShortStack entries per thread in shared memory (strided

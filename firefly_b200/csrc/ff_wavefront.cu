@@ -1072,11 +1072,13 @@ struct FrameLoop {
     cudaStream_t stream;
     uint32_t frames = 0;   // launched
     uint32_t cap;          // frames that always suffice
+    uint32_t live;         // slots that can still have a ray, at most
     // `passes` passes over each sample; a sample takes at most max_depth + 1
     // frames a pass, the next one starts in the frame that ends it, and frame
     // 0 starts the first
     FrameLoop(FFWavefrontWS* ws_, cudaStream_t stream_, const WF& w, uint32_t passes) : ws(ws_), stream(stream_)
     {
+        live = ws->P;
         const uint64_t per_slot = (w.spp + w.m - 1) / w.m;
         const uint64_t need = passes * per_slot * (w.max_depth + 1) + 1;
         FF_REQUIRE(need < (1ull << 31), "too many frames in one call");
@@ -1101,7 +1103,8 @@ struct FrameLoop {
     // running one and at most one empty frame runs at the end.
     bool next(WF& w)
     {
-        if (frames >= cap || (frames >= 2 && active_after(frames - 2) == 0)) return false;
+        if (frames >= cap) return false;
+        if (frames >= 2 && (live = active_after(frames - 2)) == 0) return false;
         w.frame = frames;
         w.first = frames == 0 ? 1u : 0u;
         w.ctr = ws->ctr_base + kCtrStride * (frames % kCtrRing);
@@ -1248,13 +1251,13 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
             FF_CUDA_CHECK(cudaStreamWaitEvent(ws->side, ws->fork, 0));
         }
         if (loop.has_rays()) {
-            ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, tctr, ws->err,
+            ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, loop.live, w.ext_hits, false, tctr, ws->err,
                                   w.ext_tag, nullptr, nullptr, scene->refracts);
             ++launches;
         }
         mark();
         if (loop.has_vertices()) {
-            ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true, tctr + 1, ws->err,
+            ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * loop.live, nullptr, true, tctr + 1, ws->err,
                                   w.sh_tag, occ, fork ? ws->side : nullptr, false,
                                   fork && defer ? kDeferShadowBlocks : 0);
             ++launches;
@@ -1490,13 +1493,13 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
             FF_CUDA_CHECK(cudaStreamWaitEvent(ws->side, ws->fork, 0));
         }
         if (loop.has_rays()) {
-            ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, P, w.ext_hits, false, tctr, ws->err, w.ext_tag,
+            ff_launch_trace_queue(ctx, bvh, w.ext_rays, w.ctr + C_EXT, loop.live, w.ext_hits, false, tctr, ws->err, w.ext_tag,
                                   nullptr, nullptr, scene->refracts);
             ++launches;
         }
         mark();
         if (loop.has_vertices()) {
-            ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * P, nullptr, true, tctr + 1, ws->err,
+            ff_launch_trace_queue(ctx, bvh, w.sh_rays, w.ctr + C_SH, 3ull * loop.live, nullptr, true, tctr + 1, ws->err,
                                   w.sh_tag, reinterpret_cast<uint8_t*>(w.ray), fork ? ws->side : nullptr);
             ++launches;
         }
