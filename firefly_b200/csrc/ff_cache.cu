@@ -2,10 +2,9 @@
 // 64-wide MLP (4 hidden ReLU layers, 3 outputs, no biases except through the
 // constant input) evaluated and trained on the fifth-generation tensor cores.
 //
-// Both kernels work on tiles of 128 records with 256 threads (8 warps):
-// thread (warp w, lane) owns row r = 32 (w % 4) + lane of the tile and half
-// h = w / 4 of its 64 columns, which is exactly the part of a 128-lane TMEM
-// accumulator its warp may read (subpartition w % 4).
+// Both kernels work on tiles of 128 records; thread (warp w, lane) owns row
+// r = 32 (w % 4) + lane of a tile, which is exactly the part of a 128-lane
+// TMEM accumulator its warp may read (subpartition w % 4).
 //   k_cache_infer  encode -> X (smem) -> 5 MMAs chains (K = 64 in four K=16
 //                  steps) with a ReLU/bf16 epilogue TMEM -> smem between
 //                  layers; activations overwrite the input tile.  Its CTA
@@ -13,7 +12,11 @@
 //                  thread per row, all 64 columns) over one copy of the
 //                  weights: while one group waits on its MMAs the others
 //                  gather hash-grid features, so the encoder's L2 gathers
-//                  overlap the tensor-core chains of the other tiles.
+//                  overlap the tensor-core chains of the other tiles.  The
+//                  gathers bound it: about 54 sectors a query from L2 (2M
+//                  queries 732 us with 80 sectors and a branch around every
+//                  fifth load, 621 us so).  With at most one tile a CTA the
+//                  groups share its encoding (4,096 records 61 -> 38 us).
 //   k_cache_train  the same forward keeping every layer's activations, the
 //                  relative-L2 loss gradient, then per layer (top down) the
 //                  weight gradient act^T * delta (M = 64, both operands
@@ -21,9 +24,18 @@
 //                  and the input gradient delta * W (W read MN-major from
 //                  the forward image); the input gradient of the hash
 //                  features is scattered to the grid's FP32 gradient.
+//                  Four threads per row (quarter h = w / 4 of the columns):
+//                  a batch of 16,384 is one tile per SM, so what counts is
+//                  the chain within a tile.  Clocks of a tile, before and
+//                  after: encoding 35,000 and 14,000 (branch-free loads,
+//                  levels dealt out evenly, twice the threads), the forward
+//                  layers with the wait for the slowest warp 19,000 and
+//                  11,000, scatter 38,000 and 31,000 (pairs of entries in one
+//                  atomic; bound by the atomics in L2).
 // Weights live in FP32 (master), their bf16 images pre-swizzled for shared
 // memory; Adam updates both.  The grid keeps FP32 features with an FP16
-// copy that the encoder reads (16 x 2^19 x 4 B = 32 MB, L2-resident).
+// copy that the encoder reads (16 x 2^19 x 4 B = 32 MB, L2-resident), the
+// coarse levels of it by cells (10 MB).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -40,7 +52,7 @@ using namespace ffu;
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;                             // training: four threads per row
 constexpr uint32_t kTileBytes = 128u * 128u;             // 128 rows x 64 bf16
 constexpr uint32_t kWBytes = 64u * 128u;                  // one 64 x 64 bf16 weight image
 constexpr uint32_t kImgBytes = kLayers * kWBytes;         // 40 KB
@@ -80,41 +92,48 @@ __device__ __forceinline__ uint4 load_chunk(const uint8_t* tile, uint32_t r, uin
     return *reinterpret_cast<const uint4*>(tile + r * 128u + (((c ^ (r & 7u)) & 7u) << 4));
 }
 
-// This thread's 32 inputs of row r: h = 0 -> columns 0..15 (levels 0..7) and
-// 32..47 (SH); h = 1 -> columns 16..31 (levels 8..15) and 48..63.
-__device__ void encode_half(const Grid& g, const Record& rec, bool valid, uint32_t h, uint32_t r, uint8_t* tile)
+// The hash features of row r, level pairs first, first + step, ... of 8 (two
+// levels: half a 16-byte chunk).  The first levels cost one load by cells, the
+// later ones five, so threads that share a row take pairs in turn.
+__device__ __forceinline__ void encode_levels(const Grid& g, const Record& rec, bool valid, uint32_t r, uint8_t* tile,
+                                              uint32_t first, uint32_t step)
 {
-    float f[32];
-    if (valid) {
-        const float3 p = normalised_pos(g, rec.px, rec.py, rec.pz);
-#pragma unroll   // all 8 levels' loads in flight (78 registers, no spills; query stage 2.39 -> 2.30 ms / 4 frames)
-        for (int j = 0; j < 8; ++j) {
-            const float2 e = level_feature(g, 8 * (int)h + j, p);
-            f[2 * j] = e.x;
-            f[2 * j + 1] = e.y;
-        }
-        if (h == 0) {
-            sh16(rec.wx, rec.wy, rec.wz, f + 16);
-        } else {
-            f[16] = rec.nx;
-            f[17] = rec.ny;
-            f[18] = rec.nz;
-            f[19] = rec.rough;
-            f[20] = 1.f;
-#pragma unroll
-            for (int k = 21; k < 32; ++k) f[k] = 0.f;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 32; ++k) f[k] = 0.f;
+    const float3 p = valid ? normalised_pos(g, rec.px, rec.py, rec.pz) : make_float3(0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (uint32_t l = 2u * first; l < (uint32_t)kLevels; l += 2u * step) {
+        float2 a, b;
+        two_features(g, (int)l, p, a, b);
+        uint2 q = make_uint2(pack_bf16(a.x, a.y), pack_bf16(b.x, b.y));
+        if (!valid) q = make_uint2(0u, 0u);
+        *reinterpret_cast<uint2*>(tile + r * 128u + ((((l >> 2) ^ (r & 7u)) & 7u) << 4) + ((l & 2u) << 2)) = q;
     }
-    store_chunk(tile, r, 2 * h, f);
-    store_chunk(tile, r, 2 * h + 1, f + 8);
-    store_chunk(tile, r, 4 + 2 * h, f + 16);
-    store_chunk(tile, r, 5 + 2 * h, f + 24);
 }
 
-// ReLU epilogue: TMEM columns [32h, 32h+32) of row r -> chunks 4h..4h+3 of dst.
+// The other 32 inputs of row r, chunk by chunk: 4 and 5 the spherical
+// harmonics, 6 normal, roughness and the constant, 7 zero.
+__device__ __forceinline__ void encode_chunk(const Record& rec, bool valid, uint32_t r, uint8_t* tile, uint32_t chunk)
+{
+    float f[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) f[k] = 0.f;
+    if (valid && chunk < 6) {
+        sh16(rec.wx, rec.wy, rec.wz, f);
+        if (chunk == 5) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) f[k] = f[8 + k];
+        }
+    } else if (valid && chunk == 6) {
+        f[0] = rec.nx;
+        f[1] = rec.ny;
+        f[2] = rec.nz;
+        f[3] = rec.rough;
+        f[4] = 1.f;
+    }
+    store_chunk(tile, r, chunk, f);
+}
+
+// ReLU epilogue: TMEM columns [32h, 32h+32) of row r -> chunks 4h..4h+3 of
+// dst, and [16h, 16h+16) -> chunks 2h, 2h + 1.
 __device__ __forceinline__ void relu_epilogue(uint32_t taddr_row, uint32_t h, uint32_t r, uint8_t* dst)
 {
     float v[32];
@@ -123,6 +142,15 @@ __device__ __forceinline__ void relu_epilogue(uint32_t taddr_row, uint32_t h, ui
     for (int k = 0; k < 32; ++k) v[k] = fmaxf(v[k], 0.f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) store_chunk(dst, r, 4 * h + c, v + 8 * c);
+}
+__device__ __forceinline__ void relu_epilogue16(uint32_t taddr_row, uint32_t h, uint32_t r, uint8_t* dst)
+{
+    float v[16];
+    tmem_ld16(taddr_row + 16u * h, v);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.f);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) store_chunk(dst, r, 2 * h + c, v + 8 * c);
 }
 
 // Copy the weight images to shared memory.
@@ -203,7 +231,7 @@ __global__ void __launch_bounds__(kInferThreads, 2) k_cache_infer(CacheArgs a)
     const bool leader = (tid & 127u) == 0;
     const uint32_t n = count_of(a);
     const uint32_t tiles = (n + kTile - 1) / kTile;
-    if (blockIdx.x * kGroups >= tiles) return;  // block-uniform, before any TMEM is held
+    if (blockIdx.x >= tiles) return;  // block-uniform, before any TMEM is held
 
     load_weights(a.w_img, w_s);
     if (tid < kGroups) mbar_init(smem_addr(mbars + tid), 1);
@@ -220,13 +248,32 @@ __global__ void __launch_bounds__(kInferThreads, 2) k_cache_infer(CacheArgs a)
     uint32_t phase = 0;
     bool failed = false;
 
-    for (uint32_t t = blockIdx.x * kGroups + g; t < tiles && !failed; t += gridDim.x * kGroups) {
+    // tiles go to the CTAs' first groups, then to their second: few tiles
+    // spread over as many SMs (each SM's L1 serves the gathers of its own)
+    // with at most one tile a CTA, all groups encode it, a third of the levels
+    // each, before the first one runs the layers
+    const bool solo = tiles <= gridDim.x;
+    if (solo) {
+        const uint32_t i = blockIdx.x * kTile + r;
+        const bool valid = i < n;
+        Record rec;
+        if (valid) rec = a.recs[i];
+        uint8_t* x = base + kImgBytes;   // the first group's tile
+        encode_levels(a.grid, rec, valid, r, x, g, kGroups);
+        for (uint32_t c = 4 + g; c < 8; c += kGroups) encode_chunk(rec, valid, r, x, c);
+        fence_smem_async();
+        __syncthreads();
+    }
+    for (uint32_t t = blockIdx.x + gridDim.x * g; t < tiles && !failed; t += gridDim.x * kGroups) {
         const uint32_t i = t * kTile + r;
         const bool valid = i < n;
         Record rec;
         if (valid) rec = a.recs[i];
-        encode_half(a.grid, rec, valid, 0, r, act);
-        encode_half(a.grid, rec, valid, 1, r, act);
+        if (!solo) {
+            encode_levels(a.grid, rec, valid, r, act, 0, 1);
+#pragma unroll
+            for (uint32_t c = 4; c < 8; ++c) encode_chunk(rec, valid, r, act, c);
+        }
         fence_smem_async();
         fence_before_sync();
         group_sync(bar);
@@ -293,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
     uint64_t* mbar_p = reinterpret_cast<uint64_t*>(dlt + kTileBytes);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(dlt + kTileBytes + 16);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t q = warp & 3u, h = warp >> 2, r = 32u * q + lane;
+    const uint32_t q = warp & 3u, h = warp >> 2, r = 32u * q + lane;   // quarter h of row r's columns
     const uint32_t mbar = smem_addr(mbar_p);
     const uint32_t n = count_of(a);
     const uint32_t tiles = (n + kTile - 1) / kTile;
@@ -336,7 +383,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
         const bool valid = i < n;
         Record rec;
         if (valid) rec = a.recs[i];
-        encode_half(a.grid, rec, valid, h, r, act[0]);
+        encode_levels(a.grid, rec, valid, r, act[0], h, 4);
+        encode_chunk(rec, valid, r, act[0], 4 + h);
         sync_out();
         // forward, keeping the activations
         for (int l = 0; l < 4 && !failed; ++l) {
@@ -345,7 +393,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
                 issue_forward(tmem, a_s[l], w0 + (uint32_t)l * kWBytes, ID_FWD);
             }
             if (!step()) { failed = true; break; }
-            relu_epilogue(trow, h, r, act[l + 1]);
+            relu_epilogue16(trow, h, r, act[l + 1]);
             sync_out();
         }
         if (failed) break;
@@ -356,6 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
         if (!step()) { failed = true; break; }
         // relative L2 loss, sum_c (y - t)^2 / (y^2 + 0.01), its gradient
         // with the denominator held constant; delta of the output layer
+        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (h == 0) {
             float y[16];
             tmem_ld16(trow, y);
@@ -370,10 +419,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
                     dy[c] = 2.f * e / den * inv_n;
                 }
             }
-            const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             store_chunk(dlt, r, 0, dy);
-            for (uint32_t c = 1; c < 8; ++c) store_chunk(dlt, r, c, zero);
+        } else {
+            store_chunk(dlt, r, 2 * h, zero);
         }
+        store_chunk(dlt, r, 2 * h + 1, zero);
         sync_out();
         // backward: layer l maps act[l] to the pre-activation whose gradient is in dlt
         for (int l = 4; l >= 0; --l) {
@@ -392,11 +442,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
             if (!step()) { failed = true; break; }
             if (l > 0) {
                 // delta of layer l: (delta W_l) * relu'(act[l])
-                float v[32];
-                tmem_ld32(trow + 32u * h, v);
+                float v[16];
+                tmem_ld16(trow + 16u * h, v);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint4 m = load_chunk(act[l], r, 4 * h + c);
+                for (int c = 0; c < 2; ++c) {
+                    const uint4 m = load_chunk(act[l], r, 2 * h + c);
                     const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -404,21 +454,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
                         if (!(av.x > 0.f)) v[8 * c + 2 * j] = 0.f;
                         if (!(av.y > 0.f)) v[8 * c + 2 * j + 1] = 0.f;
                     }
-                    store_chunk(dlt, r, 4 * h + c, v + 8 * c);
+                    store_chunk(dlt, r, 2 * h + c, v + 8 * c);
                 }
             } else {
-                // input gradient of the hash features: columns 16h..16h+15 are levels 8h..8h+7
-                float v[16];
-                tmem_ld16(trow + 16u * h, v);
+                // input gradient of the hash features: columns 8h..8h+7 are levels 4h..4h+3
+                float v[8];
+                tmem_ld8(trow + 8u * h, v);
                 if (valid) {
                     const float3 p = normalised_pos(a.grid, rec.px, rec.py, rec.pz);
-                    for (int j = 0; j < 8; ++j) {
-                        Corners c;
-                        level_corners(a.grid, 8 * (int)h + j, p, c);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int l = 4 * (int)h + j;
+                        const Cell c = level_cell(a.grid, l, p);
                         const float gx = v[2 * j], gy = v[2 * j + 1];
 #pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            atomicAdd(a.grid.grad + c.idx[k], make_float2(c.w[k] * gx, c.w[k] * gy));
+                        for (int k = 0; k < 8; k += 2) {
+                            // corners x and x + 1: where their entries are the two halves of
+                            // 16 bytes (every other x), one atomic for both
+                            const uint32_t i0 = corner_index(a.grid, l, c, k), i1 = corner_index(a.grid, l, c, k + 1);
+                            const float w0 = corner_weight(c, k), w1 = corner_weight(c, k + 1);
+                            const float2 v0 = make_float2(w0 * gx, w0 * gy), v1 = make_float2(w1 * gx, w1 * gy);
+                            if ((i0 ^ i1) == 1u) {
+                                const bool swap = i0 & 1u;
+                                const float2 lo = swap ? v1 : v0, hi = swap ? v0 : v1;
+                                atomicAdd(reinterpret_cast<float4*>(a.grid.grad + (i0 & ~1u)),
+                                          make_float4(lo.x, lo.y, hi.x, hi.y));
+                            } else {
+                                atomicAdd(a.grid.grad + i0, v0);
+                                atomicAdd(a.grid.grad + i1, v1);
+                            }
+                        }
                     }
                 }
             }
@@ -430,13 +495,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_cache_train(CacheArgs a)
         // weight gradients: accumulator l holds act[l]^T delta, rows m = input
         // unit (M = 64: TMEM lanes 0-15 of each subpartition), columns n
         for (int l = 0; l < kLayers; ++l) {
-            float v[32];
-            tmem_ld32(trow + 64u + 64u * (uint32_t)l + 32u * h, v);
+            float v[16];
+            tmem_ld16(trow + 64u + 64u * (uint32_t)l + 16u * h, v);
             if (lane < 16) {
                 const uint32_t m = 16u * q + lane;
                 float* gw = a.grad_w + (size_t)l * kWidth * kWidth;
-                for (int j = 0; j < 32; ++j) {
-                    const uint32_t nn = 32u * h + (uint32_t)j;
+                for (int j = 0; j < 16; ++j) {
+                    const uint32_t nn = 16u * h + (uint32_t)j;
                     if (l == kLayers - 1 && nn >= (uint32_t)kOutputs) break;
                     atomicAdd(gw + nn * kWidth + m, v[j]);
                 }
@@ -517,9 +582,34 @@ __global__ void k_adam_mlp(float* __restrict__ w, float* __restrict__ g, float* 
     put_image(img, i, wi);
 }
 
+// Writes entry i (half precision) to the cells around it, where its level is
+// also kept by cells (Grid::cells): each of up to 8 cells has it as another corner.
+__device__ __forceinline__ void put_cells(const Grid& g, uint32_t* __restrict__ cells, uint32_t i, __half2 value)
+{
+    const uint32_t l = i >> g.log2_T;
+    if (l >= g.cell_levels) return;
+    const uint32_t side = g.dense_side[l], n = side - 1u;
+    const uint32_t j = i & ((1u << g.log2_T) - 1u);
+    const uint32_t x = j % side, y = (j / side) % side, z = j / (side * side);
+    if (z > n) return;   // past the level's last entry
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t cx = x - (k & 1u), cy = y - ((k >> 1) & 1u), cz = z - (k >> 2);   // (wraps below 0)
+        if (cx < n && cy < n && cz < n)
+            cells[8 * (size_t)(g.cell_off[l] + cx + n * (cy + n * cz)) + k] = *reinterpret_cast<uint32_t*>(&value);
+    }
+}
+
+__global__ void k_cells(Grid g, uint32_t* __restrict__ cells, const __half2* __restrict__ table_h)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < g.cell_levels << g.log2_T) put_cells(g, cells, i, table_h[i]);
+}
+
 // Sparse Adam over the grid: entries no record touched keep their state.
 __global__ void k_adam_grid(float2* __restrict__ table, __half2* __restrict__ table_h, float2* __restrict__ g,
-                            float2* __restrict__ m, float2* __restrict__ v, uint32_t n, AdamHP hp)
+                            float2* __restrict__ m, float2* __restrict__ v, uint32_t n, AdamHP hp, Grid grid,
+                            uint32_t* __restrict__ cells)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -536,7 +626,9 @@ __global__ void k_adam_grid(float2* __restrict__ table, __half2* __restrict__ ta
     m[i] = mi;
     v[i] = vi;
     table[i] = p;
-    table_h[i] = __floats2half2_rn(p.x, p.y);
+    const __half2 h = __floats2half2_rn(p.x, p.y);
+    table_h[i] = h;
+    put_cells(grid, cells, i, h);
 }
 
 __global__ void k_half_of(const float2* __restrict__ table, __half2* __restrict__ table_h, uint32_t n)
@@ -569,6 +661,27 @@ void ff_cache_setup_grid(ff_cache* c)
         const uint64_t side = (uint64_t)cells + 1;
         g.dense_side[l] = side * side * side <= T ? (uint32_t)side : 0u;
     }
+    // the leading dense levels also by cells (their resolutions never fall)
+    uint64_t total = 0;
+    g.cell_levels = 0;
+    for (int l = 0; l < kLevels; ++l) {
+        const uint64_t cells = (uint64_t)g.scale[l], n = cells * cells * cells;
+        if (!g.dense_side[l] || n > kCellMax) break;
+        g.cell_off[l] = (uint32_t)total;
+        total += n;
+        g.cell_levels = (uint32_t)l + 1u;
+    }
+    c->cells.alloc(32 * total);
+    g.cells = c->cells.as<uint4>();
+}
+
+// The cells' copy of the half-precision table, from scratch.
+static void fill_cells(ff_cache* c, cudaStream_t st)
+{
+    const Grid& g = c->grid;
+    if (!g.cell_levels) return;
+    k_cells<<<grid_for((size_t)g.cell_levels << g.log2_T, 256), 256, 0, st>>>(g, c->cells.as<uint32_t>(),
+                                                                              c->table_h.as<__half2>());
 }
 
 void ff_cache_init_params(ff_cache* c)
@@ -576,6 +689,7 @@ void ff_cache_init_params(ff_cache* c)
     cudaStream_t st = c->ctx->stream;
     const uint32_t n = kLevels << c->prm.log2_table_size;
     k_init_grid<<<grid_for(n, 256), 256, 0, st>>>(c->table.as<float2>(), c->table_h.as<__half2>(), n, c->prm.seed);
+    fill_cells(c, st);
     k_init_mlp<<<grid_for(kParams, 256), 256, 0, st>>>(c->mlp.as<float>(), c->prm.seed);
     k_pack_mlp<<<grid_for(kParams, 256), 256, 0, st>>>(c->mlp.as<float>(), c->mlp_img.as<uint8_t>());
     FF_CUDA_CHECK(cudaMemsetAsync(c->grid_grad.ptr, 0, sizeof(float2) * n, st));
@@ -623,7 +737,7 @@ void ff_cache_launch_infer(ff_cache* c, const void* recs, uint32_t n_max, const 
     a.out_rgb = out_rgb;
     a.frame = frame;
     const uint32_t tiles = (n_max + kTile - 1) / kTile;
-    const uint32_t grid = std::min<uint32_t>((tiles + kGroups - 1) / kGroups, (uint32_t)c->ctx->num_sms * 2u);
+    const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)c->ctx->num_sms * 2u);
     k_cache_infer<<<grid, kInferThreads, kInferSmem, c->ctx->stream>>>(a);
     FF_CUDA_CHECK(cudaGetLastError());
 }
@@ -658,7 +772,7 @@ static void launch_train(ff_cache* c, const Record* recs, uint32_t offset, uint3
     const uint32_t ng = kLevels << c->prm.log2_table_size;
     k_adam_grid<<<grid_for(ng, 256), 256, 0, st>>>(c->table.as<float2>(), c->table_h.as<__half2>(),
                                                   c->grid_grad.as<float2>(), c->grid_m.as<float2>(),
-                                                  c->grid_v.as<float2>(), ng, hp);
+                                                  c->grid_v.as<float2>(), ng, hp, c->grid, c->cells.as<uint32_t>());
     FF_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -678,6 +792,7 @@ void ff_cache_refresh_copies(ff_cache* c)
     cudaStream_t st = c->ctx->stream;
     const uint32_t n = kLevels << c->prm.log2_table_size;
     k_half_of<<<grid_for(n, 256), 256, 0, st>>>(c->table.as<float2>(), c->table_h.as<__half2>(), n);
+    fill_cells(c, st);
     k_pack_mlp<<<grid_for(kParams, 256), 256, 0, st>>>(c->mlp.as<float>(), c->mlp_img.as<uint8_t>());
     FF_CUDA_CHECK(cudaGetLastError());
 }

@@ -29,7 +29,14 @@ struct Grid {
     float3 lo, inv_ext;             // position normalisation (scene box)
     float scale[kLevels];           // cells per unit cube side at each level
     uint32_t dense_side[kLevels];   // side+1 of a densely indexed level, 0 for hashed levels
+    // The first cell_levels levels (dense ones of at most kCellMax cells) once
+    // more, by cells: the 8 corner entries of a cell in one 32-byte sector, the
+    // cells of level l from cell_off[l], x fastest.
+    const uint4* cells;
+    uint32_t cell_levels;
+    uint32_t cell_off[kLevels];
 };
+constexpr uint32_t kCellMax = 1u << 18;   // cells of a level kept by cells (8 MB)
 
 // One record: a vertex (position, roughness, outgoing direction, normal)
 // and a value (training: target radiance; render queries: path throughput).
@@ -72,14 +79,12 @@ __device__ __forceinline__ float3 normalised_pos(const Grid& g, float px, float 
     return p;
 }
 
-// The 8 corners of the level-l cell holding p: table indices and trilinear
-// weights (corner bit 0 = +x, bit 1 = +y, bit 2 = +z).
-struct Corners {
-    uint32_t idx[8];
-    float w[8];
+// The level-l cell holding p and p's place in it.
+struct Cell {
+    uint32_t x, y, z;
+    float tx, ty, tz;
 };
-
-__device__ __forceinline__ void level_corners(const Grid& g, int l, float3 p, Corners& c)
+__device__ __forceinline__ Cell level_cell(const Grid& g, int l, float3 p)
 {
     const float s = g.scale[l];
     const float fx = p.x * s, fy = p.y * s, fz = p.z * s;
@@ -88,21 +93,24 @@ __device__ __forceinline__ void level_corners(const Grid& g, int l, float3 p, Co
     ix = max(ix, 0);
     iy = max(iy, 0);
     iz = max(iz, 0);
-    const float tx = fminf(fmaxf(fx - (float)ix, 0.f), 1.f);
-    const float ty = fminf(fmaxf(fy - (float)iy, 0.f), 1.f);
-    const float tz = fminf(fmaxf(fz - (float)iz, 0.f), 1.f);
+    Cell c;
+    c.x = (uint32_t)ix, c.y = (uint32_t)iy, c.z = (uint32_t)iz;
+    c.tx = fminf(fmaxf(fx - (float)ix, 0.f), 1.f);
+    c.ty = fminf(fmaxf(fy - (float)iy, 0.f), 1.f);
+    c.tz = fminf(fmaxf(fz - (float)iz, 0.f), 1.f);
+    return c;
+}
+// Trilinear weight and table index of corner k (bit 0 = +x, bit 1 = +y, bit 2 = +z).
+__device__ __forceinline__ float corner_weight(const Cell& c, int k)
+{
+    return ((k & 1) ? c.tx : 1.f - c.tx) * (((k >> 1) & 1) ? c.ty : 1.f - c.ty) * ((k >> 2) ? c.tz : 1.f - c.tz);
+}
+__device__ __forceinline__ uint32_t corner_index(const Grid& g, int l, const Cell& c, int k)
+{
+    const uint32_t x = c.x + (k & 1), y = c.y + ((k >> 1) & 1), z = c.z + (k >> 2);
     const uint32_t side = g.dense_side[l];
-    const uint32_t mask = (1u << g.log2_T) - 1u;
-    const uint32_t base = (uint32_t)l << g.log2_T;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t x = (uint32_t)ix + (k & 1), y = (uint32_t)iy + ((k >> 1) & 1), z = (uint32_t)iz + (k >> 2);
-        uint32_t i;
-        if (side) i = x + side * (y + side * z);
-        else i = (x * 1u) ^ (y * 2654435761u) ^ (z * 805459861u);
-        c.idx[k] = base + (i & mask);
-        c.w[k] = ((k & 1) ? tx : 1.f - tx) * (((k >> 1) & 1) ? ty : 1.f - ty) * ((k >> 2) ? tz : 1.f - tz);
-    }
+    const uint32_t i = side ? x + side * (y + side * z) : (x * 1u) ^ (y * 2654435761u) ^ (z * 805459861u);
+    return ((uint32_t)l << g.log2_T) + (i & ((1u << g.log2_T) - 1u));
 }
 
 // Entry j (0..3) of four packed half2 entries.
@@ -117,30 +125,91 @@ __device__ __forceinline__ float2 half2_bits(uint32_t u)
     return __half22float2(h);
 }
 
-// Trilinear feature of level l at p.  Corners k (x) and k + 1 (x + 1) share
-// y and z, so their entries usually sit in one aligned group of four: on a
-// dense level they are neighbours, and on a hashed level x enters the hash
-// by XOR, so the two indices differ in the bits of x ^ (x + 1), which stay
-// below 4 three times in four.  The group is one 16-byte load (one sector
-// per lane instead of two); an entry outside it is read alone.  The sum runs
-// over the corners in the same order, so the feature is unchanged.
-__device__ __forceinline__ float2 level_feature(const Grid& g, int l, float3 p)
+// The table entries of one level's 8 corners, loaded without branches, so that
+// the loads of several levels are in flight together.
+//
+// By cells, one 32-byte load.  Else corners k (x) and k + 1 (x + 1) share y
+// and z, so their entries usually sit in one aligned group of four: on a
+// dense level they are neighbours, and on a hashed level x enters the hash by
+// XOR, so the two indices differ in the bits of x ^ (x + 1), which stay below
+// 4 three times in four.  The group is one 16-byte load (one sector per lane
+// instead of two); an entry outside it is read alone, by a predicated load.
+// With a branch around that load every level's four pairs waited for one
+// another: 16 levels took 100,000 cycles in a launch of one tile per SM.
+struct CornerEntries {
+    uint32_t e[8];
+};
+__device__ __forceinline__ CornerEntries cell_entries(const Grid& g, int l, const Cell& c)
 {
-    Corners c;
-    level_corners(g, l, p, c);
+    const uint32_t n = (uint32_t)g.scale[l];
+    const uint4* p = g.cells + 2 * (size_t)(g.cell_off[l] + c.x + n * (c.y + n * c.z));
+    CornerEntries r;
+    asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r.e[0]), "=r"(r.e[1]), "=r"(r.e[2]), "=r"(r.e[3]), "=r"(r.e[4]), "=r"(r.e[5]), "=r"(r.e[6]), "=r"(r.e[7])
+        : "l"(p));
+    return r;
+}
+struct PairLoads {
+    uint4 q[4];
+    uint32_t alone[4], i0[4], i1[4];
+};
+__device__ __forceinline__ PairLoads load_pairs(const Grid& g, int l, const Cell& c)
+{
+    PairLoads r;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        r.i0[k] = corner_index(g, l, c, 2 * k);
+        r.i1[k] = corner_index(g, l, c, 2 * k + 1);
+        r.q[k] = __ldg(reinterpret_cast<const uint4*>(g.table_h + (r.i0[k] & ~3u)));
+        asm("{\n\t.reg .pred p;\n\t"
+            "setp.ge.u32 p, %2, 4;\n\t"
+            "mov.b32 %0, 0;\n\t"
+            "@p ld.global.nc.b32 %0, [%1];\n\t}"
+            : "=r"(r.alone[k])
+            : "l"(g.table_h + r.i1[k]), "r"(r.i0[k] ^ r.i1[k]));
+    }
+    return r;
+}
+__device__ __forceinline__ CornerEntries pair_entries(const PairLoads& a)
+{
+    CornerEntries r;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        r.e[2 * k] = pick4(a.q[k], a.i0[k] & 3u);
+        r.e[2 * k + 1] = (a.i0[k] ^ a.i1[k]) < 4u ? pick4(a.q[k], a.i1[k] & 3u) : a.alone[k];
+    }
+    return r;
+}
+// Trilinear feature: the sum over the corners in order.
+__device__ __forceinline__ float2 blend(const Cell& c, const CornerEntries& e)
+{
     float2 f = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 0; k < 8; k += 2) {
-        const uint32_t i0 = c.idx[k], i1 = c.idx[k + 1];
-        const uint4 q = *reinterpret_cast<const uint4*>(g.table_h + (i0 & ~3u));
-        const uint32_t b1 = (i0 ^ i1) < 4u ? pick4(q, i1 & 3u) : *reinterpret_cast<const uint32_t*>(g.table_h + i1);
-        const float2 e0 = half2_bits(pick4(q, i0 & 3u)), e1 = half2_bits(b1);
-        f.x += c.w[k] * e0.x;
-        f.y += c.w[k] * e0.y;
-        f.x += c.w[k + 1] * e1.x;
-        f.y += c.w[k + 1] * e1.y;
+    for (int k = 0; k < 8; ++k) {
+        const float w = corner_weight(c, k);
+        const float2 v = half2_bits(e.e[k]);
+        f.x += w * v.x;
+        f.y += w * v.y;
     }
     return f;
+}
+// The features of levels l and l + 1 at p.
+__device__ __forceinline__ void two_features(const Grid& g, int l, float3 p, float2& fa, float2& fb)
+{
+    const Cell ca = level_cell(g, l, p), cb = level_cell(g, l + 1, p);
+    if (l + 1 < (int)g.cell_levels) {
+        const CornerEntries a = cell_entries(g, l, ca), b = cell_entries(g, l + 1, cb);
+        fa = blend(ca, a);
+        fb = blend(cb, b);
+    } else if (l < (int)g.cell_levels) {
+        const CornerEntries a = cell_entries(g, l, ca);
+        const PairLoads b = load_pairs(g, l + 1, cb);
+        fa = blend(ca, a);
+        fb = blend(cb, pair_entries(b));
+    } else {
+        fa = blend(ca, pair_entries(load_pairs(g, l, ca)));
+        fb = blend(cb, pair_entries(load_pairs(g, l + 1, cb)));
+    }
 }
 
 // Real spherical harmonics of degree 0..3 (16 functions) of the unit

@@ -295,6 +295,7 @@ struct ff_cache {
     float3 lo{0, 0, 0}, hi{0, 0, 0};  // scene box
     ffc::Grid grid{};
     DevBuf table, table_h, grid_grad, grid_m, grid_v;   // float2 / half2 per grid entry
+    DevBuf cells;         // the first levels' half2 entries by cells (Grid::cells)
     DevBuf mlp, mlp_img, mlp_grad, mlp_m, mlp_v;        // FP32 weights, their bf16 images, Adam state
     DevBuf loss;          // float: sum of training losses since the last reset of the counter
     DevBuf err;           // uint32: tensor-core waits that gave up
