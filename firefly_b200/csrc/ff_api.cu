@@ -6,8 +6,11 @@
 #include <algorithm>
 #include <cstring>
 #include <new>
+#include <utility>
+#include <vector>
 
 #include "ff_internal.h"
+#include "ff_shade.cuh"
 
 namespace {
 
@@ -47,10 +50,46 @@ struct DeviceGuard {
     }
 };
 
-void upload(DevBuf& b, const void* host, size_t bytes, cudaStream_t st)
+// One allocation for the scene's buffers, at the sizes the description gives.
+// (The tangent frames are allocated where a normal texture asks for them.)
+void place_scene(ff_scene* s, const ff_scene_desc* d)
 {
-    b.alloc(bytes);
-    if (bytes) FF_CUDA_CHECK(cudaMemcpyAsync(b.ptr, host, bytes, cudaMemcpyHostToDevice, st));
+    std::vector<std::pair<DevBuf*, size_t>> parts;
+    const size_t n = d->num_triangles;
+    if (n) {
+        parts.push_back({&s->nodes, sizeof(FFNode8) * (n / 2 + 2)});
+        parts.push_back({&s->tris, sizeof(FFTri) * n});
+        parts.push_back({&s->shade, sizeof(FFShadeTri) * n});
+    }
+    parts.push_back({&s->materials, sizeof(ff_material) * std::max<size_t>(1, d->num_materials)});
+    for (uint32_t i = 0; i < d->num_textures; ++i) {
+        const ff_texture_desc& td = d->textures[i];
+        FF_REQUIRE(td.rgb && td.width > 0 && td.height > 0, "texture without texels");
+        s->textures.push_back(new DevBuf());
+        parts.push_back({s->textures.back(), sizeof(float3) * td.width * td.height});
+    }
+    parts.push_back({&s->tex_table, sizeof(FFTexView) * d->num_textures});
+    parts.push_back({&s->area_lights, sizeof(ff_area_light) * d->num_area_lights});
+    parts.push_back({&s->dir_lights, sizeof(ff_directional_light) * d->num_directional_lights});
+    if (d->env_rgb) {
+        const size_t w = d->env_width, h = d->env_height;
+        FFEnvLight& e = s->env;
+        parts.push_back({&e.rgb, sizeof(float3) * w * h});
+        parts.push_back({&e.marginal, sizeof(double) * h});
+        parts.push_back({&e.conditional, sizeof(double) * w * h});
+        parts.push_back({&e.pdf, sizeof(float) * w * h});
+        parts.push_back({&e.denom, sizeof(double) * 2});
+        parts.push_back({&e.texel4, sizeof(float4) * w * h});
+        parts.push_back({&e.guide, sizeof(uint32_t) * ((size_t)kGuideMarginal + 1 + h * ((size_t)kGuideCond + 1))});
+    }
+    size_t total = 0;
+    for (auto& p : parts) total += (p.second + 255) & ~size_t(255);
+    s->arena.alloc(total);
+    char* at = s->arena.as<char>();
+    for (auto& p : parts) {
+        p.first->place(at, p.second);
+        at += (p.second + 255) & ~size_t(255);
+    }
 }
 
 }  // namespace
@@ -116,6 +155,9 @@ ff_status ff_context_destroy(ff_context* ctx)
         ctx->counters.release();
         ctx->io_rays.release();
         ctx->io_hits.release();
+        ctx->io_small.release();
+        ctx->scratch.release();
+        if (ctx->io_pin) cudaFreeHost(ctx->io_pin);
         for (auto& b : ctx->adj_io) b.release();
         if (ctx->io_in) cudaStreamSynchronize(ctx->io_in);
         if (ctx->io_out) cudaStreamSynchronize(ctx->io_out);
@@ -163,12 +205,14 @@ ff_status ff_scene_create(ff_context* ctx, const ff_scene_desc* d, ff_scene** ou
         FF_REQUIRE(d->num_triangles == 0 || (d->positions && d->indices), "positions and indices are required");
         FF_REQUIRE(d->num_triangles == 0 || d->num_vertices > 0, "num_vertices must be > 0");
         FF_REQUIRE(d->num_triangles < (1u << 30), "too many triangles");
-        for (uint64_t i = 0; i < 3ull * d->num_triangles; ++i)
-            FF_REQUIRE(d->indices[i] < d->num_vertices, "triangle index out of range");
+        uint32_t largest = 0;
+        for (uint64_t i = 0; i < 3ull * d->num_triangles; ++i) largest = std::max(largest, d->indices[i]);
+        FF_REQUIRE(d->num_triangles == 0 || largest < d->num_vertices, "triangle index out of range");
         if (d->material_ids) {
-            for (uint32_t i = 0; i < d->num_triangles; ++i)
-                FF_REQUIRE(d->material_ids[i] < (d->num_materials ? d->num_materials : 1u),
-                           "material id out of range");
+            largest = 0;
+            for (uint32_t i = 0; i < d->num_triangles; ++i) largest = std::max(largest, d->material_ids[i]);
+            FF_REQUIRE(d->num_triangles == 0 || largest < (d->num_materials ? d->num_materials : 1u),
+                       "material id out of range");
         }
         FF_REQUIRE(d->num_materials < (1u << 24), "at most 2^24 - 1 materials");
         for (uint32_t m = 0; m < d->num_materials; ++m) {
@@ -182,12 +226,15 @@ ff_status ff_scene_create(ff_context* ctx, const ff_scene_desc* d, ff_scene** ou
         FF_REQUIRE(d->num_area_lights == 0 || d->area_lights, "area_lights is NULL");
         FF_REQUIRE(d->num_directional_lights == 0 || d->directional_lights, "directional_lights is NULL");
         cudaStream_t stream = ctx->stream;
-        DevBuf pos, idx;
-        upload(pos, d->positions, sizeof(float) * 3ull * d->num_vertices, stream);
-        upload(idx, d->indices, sizeof(uint32_t) * 3ull * d->num_triangles, stream);
-        ff_build_bvh(ctx, s, pos.as<float3>(), idx.as<uint3>(), d->num_triangles);
+        place_scene(s, d);
+        FFTemp temp(ctx);
+        float3* pos = temp.get<float3>(d->num_vertices);
+        uint3* idx = temp.get<uint3>(d->num_triangles);
+        if (pos) FF_CUDA_CHECK(cudaMemcpyAsync(pos, d->positions, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, stream));
+        if (idx) FF_CUDA_CHECK(cudaMemcpyAsync(idx, d->indices, sizeof(uint3) * d->num_triangles, cudaMemcpyHostToDevice, stream));
+        ff_build_bvh(ctx, s, pos, idx, d->num_triangles);
         FF_REQUIRE(s->depth <= (uint32_t)kMaxStackDepth, "BVH deeper than the traversal stack");
-        ff_build_shading(ctx, s, d, pos.as<float3>(), idx.as<uint3>());
+        ff_build_shading(ctx, s, d, pos, idx);
         s->camera = d->camera;
         FF_CUDA_CHECK(cudaStreamSynchronize(stream));
     });
@@ -260,6 +307,36 @@ namespace {
 // Rays per chunk of a host-pointer trace: 64 MB in, 32 MB out.
 constexpr uint64_t kIoChunk = 1ull << 21;
 
+// Host-pointer traces of up to this many rays go through pinned staging.
+constexpr uint64_t kIoSmall = 8192;
+
+// A small host-pointer trace: one copy in (the zeroed ray counter, the rays,
+// the zeroed error count), the trace, one copy out (the error count, the
+// hits), through pinned staging that the context keeps.  Three copies from
+// and to pageable memory, a memset and two more streams' events took 67 us
+// for 100 rays, this 45.  Synchronous; returns the error count.
+unsigned int trace_host_small(ff_context* ctx, const ff_scene* s, const ff_ray* rays, uint64_t n, ff_hit* hits, bool any,
+                              bool two)
+{
+    constexpr size_t kBytes = 32 + kIoSmall * (sizeof(ff_ray) + sizeof(ff_hit));
+    ctx->io_small.alloc(kBytes);
+    if (!ctx->io_pin) FF_CUDA_CHECK(cudaMallocHost(&ctx->io_pin, kBytes));
+    char *pin = ctx->io_pin, *dev = ctx->io_small.as<char>();
+    const size_t at_err = 16 + n * sizeof(ff_ray), at_hits = at_err + 16;
+    std::memset(pin, 0, 16);
+    std::memcpy(pin + 16, rays, n * sizeof(ff_ray));
+    std::memset(pin + at_err, 0, 16);
+    FF_CUDA_CHECK(cudaMemcpyAsync(dev, pin, at_hits, cudaMemcpyHostToDevice, ctx->stream));
+    ff_launch_trace_scratch(ctx, s, reinterpret_cast<ff_ray*>(dev + 16), n, reinterpret_cast<ff_hit*>(dev + at_hits), any,
+                            reinterpret_cast<unsigned long long*>(dev), reinterpret_cast<unsigned int*>(dev + at_err), two);
+    FF_CUDA_CHECK(cudaMemcpyAsync(pin + at_err, dev + at_err, 16 + n * sizeof(ff_hit), cudaMemcpyDeviceToHost, ctx->stream));
+    FF_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    unsigned int err;
+    std::memcpy(&err, pin + at_err, sizeof(err));
+    std::memcpy(hits, pin + at_hits, n * sizeof(ff_hit));
+    return err;
+}
+
 // The host-pointer trace as a three-stage pipeline over chunks: the copy in
 // of chunk i + 1 (io_in) and the copy out of chunk i - 1 (io_out) run beside
 // the trace of chunk i (the context's stream), so both copy directions are
@@ -329,6 +406,9 @@ ff_status ff_trace(ff_context* ctx, const ff_scene* s, const ff_ray* rays, uint6
             FF_REQUIRE((reinterpret_cast<uintptr_t>(rays) & 15) == 0 && (reinterpret_cast<uintptr_t>(hits) & 15) == 0,
                        "device rays and hits must be 16-byte aligned");
             ff_launch_trace(ctx, s, rays, n, hits, any, two);
+        } else if (n <= kIoSmall) {
+            if (trace_host_small(ctx, s, rays, n, hits, any, two))
+                throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
         } else {
             ctx->io_rays.alloc(sizeof(ff_ray) * n);
             ctx->io_hits.alloc(sizeof(ff_hit) * n);

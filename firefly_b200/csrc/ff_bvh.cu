@@ -618,47 +618,46 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
     FF_CUDA_CHECK(cudaEventCreate(&e1));
     FF_CUDA_CHECK(cudaEventRecord(e0, st));
 
-    DevBuf rec, blo, bhi, cen, keys, keys2, vals, vals2, bin, plan, pint, pleaf, arrivals, qa, qb, misc, temp;
-    rec.alloc(sizeof(FFTri) * n);
-    blo.alloc(sizeof(float3) * n);
-    bhi.alloc(sizeof(float3) * n);
-    cen.alloc(sizeof(float3) * n);
-    keys.alloc(sizeof(uint64_t) * n);
-    keys2.alloc(sizeof(uint64_t) * n);
-    vals.alloc(sizeof(uint32_t) * n);
-    vals2.alloc(sizeof(uint32_t) * n);
-    misc.alloc(64 * sizeof(uint32_t));
-    uint32_t* counters = misc.as<uint32_t>();
+    FFTemp temp(ctx);
+    FFTri* rec = temp.get<FFTri>(n);
+    float3* blo = temp.get<float3>(n);
+    float3* bhi = temp.get<float3>(n);
+    float3* cen = temp.get<float3>(n);
+    uint64_t* keys = temp.get<uint64_t>(n);
+    uint64_t* keys2 = temp.get<uint64_t>(n);
+    uint32_t* vals = temp.get<uint32_t>(n);
+    uint32_t* vals2 = temp.get<uint32_t>(n);
+    uint32_t* counters = temp.get<uint32_t>(64);
     int* cb = reinterpret_cast<int*>(counters + 16);
 
     const int B = 256;
     const uint32_t G = (n + B - 1) / B;
     k_init_counters<<<1, 1, 0, st>>>(cb);
-    k_prep<<<G, B, 0, st>>>(d_pos, d_idx, n, rec.as<FFTri>(), blo.as<float3>(), bhi.as<float3>(),
-                            cen.as<float3>(), cb, cb + 12);
-    k_morton<<<G, B, 0, st>>>(cen.as<float3>(), n, cb, keys.as<uint64_t>(), vals.as<uint32_t>(), blo.as<float3>(),
-                              bhi.as<float3>());
+    k_prep<<<G, B, 0, st>>>(d_pos, d_idx, n, rec, blo, bhi,
+                            cen, cb, cb + 12);
+    k_morton<<<G, B, 0, st>>>(cen, n, cb, keys, vals, blo,
+                              bhi);
     size_t temp_bytes = 0;
-    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys.as<uint64_t>(), keys2.as<uint64_t>(),
-                                                  vals.as<uint32_t>(), vals2.as<uint32_t>(), (int)n, 0, 64, st));
-    temp.alloc(std::max<size_t>(temp_bytes, 16));
-    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(temp.ptr, temp_bytes, keys.as<uint64_t>(), keys2.as<uint64_t>(),
-                                                  vals.as<uint32_t>(), vals2.as<uint32_t>(), (int)n, 0, 64, st));
-    const uint64_t* skeys = keys2.as<uint64_t>();
-    const uint32_t* order = vals2.as<uint32_t>();
+    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys2,
+                                                  vals, vals2, (int)n, 0, 64, st));
+    void* sort_temp = temp.get<char>(std::max<size_t>(temp_bytes, 16));
+    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_temp, temp_bytes, keys, keys2,
+                                                  vals, vals2, (int)n, 0, 64, st));
+    const uint64_t* skeys = keys2;
+    const uint32_t* order = vals2;
 
     uint32_t n_int = n > 1 ? n - 1 : 1;
-    bin.alloc(sizeof(BinNode) * n_int);
-    plan.alloc(sizeof(WidePlan) * n_int);
-    pint.alloc(sizeof(int32_t) * n_int);
-    pleaf.alloc(sizeof(int32_t) * n);
-    arrivals.alloc(sizeof(uint32_t) * n_int);
-    FF_CUDA_CHECK(cudaMemsetAsync(arrivals.ptr, 0, sizeof(uint32_t) * n_int, st));
+    BinNode* bin = temp.get<BinNode>(n_int);
+    WidePlan* plan = temp.get<WidePlan>(n_int);
+    int32_t* pint = temp.get<int32_t>(n_int);
+    int32_t* pleaf = temp.get<int32_t>(n);
+    uint32_t* arrivals = temp.get<uint32_t>(n_int);
+    FF_CUDA_CHECK(cudaMemsetAsync(arrivals, 0, sizeof(uint32_t) * n_int, st));
     if (n > 1) {
-        k_radix_tree<<<(n - 1 + B - 1) / B, B, 0, st>>>(skeys, (int)n, bin.as<BinNode>(), pint.as<int32_t>(),
-                                                       pleaf.as<int32_t>());
-        k_bounds_up<<<G, B, 0, st>>>((int)n, order, blo.as<float3>(), bhi.as<float3>(), bin.as<BinNode>(),
-                                     plan.as<WidePlan>(), pint.as<int32_t>(), pleaf.as<int32_t>(), arrivals.as<uint32_t>());
+        k_radix_tree<<<(n - 1 + B - 1) / B, B, 0, st>>>(skeys, (int)n, bin, pint,
+                                                       pleaf);
+        k_bounds_up<<<G, B, 0, st>>>((int)n, order, blo, bhi, bin,
+                                     plan, pint, pleaf, arrivals);
     }
 
     // Wide nodes: about n / 7.  The plan may give a node as few as two
@@ -669,20 +668,18 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
     uint32_t host_counters[4];
     for (uint32_t max_wide : {n / 2 + 2, n + 1}) {
         s->nodes.alloc(sizeof(FFNode8) * max_wide);
-        qa.alloc(sizeof(CollapseItem) * max_wide);
-        qb.alloc(sizeof(CollapseItem) * max_wide);
+        CollapseItem* qin = temp.get<CollapseItem>(max_wide);
+        CollapseItem* qout = temp.get<CollapseItem>(max_wide);
         k_reset_collapse<<<1, 1, 0, st>>>(counters);
         CollapseItem root{n > 1 ? 0 : ~0, 0u};
-        FF_CUDA_CHECK(cudaMemcpyAsync(qa.ptr, &root, sizeof(root), cudaMemcpyHostToDevice, st));
-        CollapseItem* qin = qa.as<CollapseItem>();
-        CollapseItem* qout = qb.as<CollapseItem>();
+        FF_CUDA_CHECK(cudaMemcpyAsync(qin, &root, sizeof(root), cudaMemcpyHostToDevice, st));
         host_counters[3] = 0;
         depth = 0;
         for (uint32_t n_in = 1; n_in > 0 && !host_counters[3]; std::swap(qin, qout)) {
             FF_CUDA_CHECK(cudaMemsetAsync(counters, 0, sizeof(uint32_t), st));
             k_collapse<<<(n_in + 127) / 128, 128, 0, st>>>(
-                qin, n_in, qout, counters, max_wide, n, bin.as<BinNode>(), plan.as<WidePlan>(), order, blo.as<float3>(),
-                bhi.as<float3>(), rec.as<FFTri>(), s->nodes.as<FFNode8>(), s->tris.as<FFTri>());
+                qin, n_in, qout, counters, max_wide, n, bin, plan, order, blo,
+                bhi, rec, s->nodes.as<FFNode8>(), s->tris.as<FFTri>());
             FF_CUDA_CHECK(cudaMemcpyAsync(host_counters, counters, sizeof(host_counters), cudaMemcpyDeviceToHost, st));
             FF_CUDA_CHECK(cudaStreamSynchronize(st));
             ++depth;
@@ -701,13 +698,12 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
     if (host_counters[2] != n) throw FFError{FF_ERR_INTERNAL, "BVH collapse lost triangles"};
     s->num_nodes = host_counters[1];
     {
-        DevBuf refs;
-        refs.alloc(sizeof(uint32_t) * (n + 1));
-        uint32_t* d_err = refs.as<uint32_t>() + n;
-        FF_CUDA_CHECK(cudaMemsetAsync(refs.ptr, 0, sizeof(uint32_t) * (n + 1), st));
+        uint32_t* refs = temp.get<uint32_t>((size_t)n + 1);
+        uint32_t* d_err = refs + n;
+        FF_CUDA_CHECK(cudaMemsetAsync(refs, 0, sizeof(uint32_t) * (n + 1), st));
         k_validate<<<(s->num_nodes + 127) / 128, 128, 0, st>>>(s->nodes.as<FFNode8>(), s->num_nodes,
-                                                              s->tris.as<FFTri>(), n, refs.as<uint32_t>(), d_err);
-        k_validate_refs<<<G, B, 0, st>>>(refs.as<uint32_t>(), n, d_err);
+                                                              s->tris.as<FFTri>(), n, refs, d_err);
+        k_validate_refs<<<G, B, 0, st>>>(refs, n, d_err);
         uint32_t h_err = 0;
         FF_CUDA_CHECK(cudaMemcpyAsync(&h_err, d_err, sizeof(h_err), cudaMemcpyDeviceToHost, st));
         FF_CUDA_CHECK(cudaStreamSynchronize(st));

@@ -183,14 +183,14 @@ void ff_build_env_tables(ff_context* ctx, ff_scene* s)
     e.conditional.alloc(sizeof(double) * (size_t)w * h);
     e.pdf.alloc(sizeof(float) * (size_t)w * h);
     e.denom.alloc(sizeof(double) * 2);
-    DevBuf lum, rows, mp;
-    lum.alloc(sizeof(float) * (size_t)w * h);
-    rows.alloc(sizeof(double) * h);
-    mp.alloc(sizeof(double) * h);
-    k_env_rows<<<h, kEnvBlock, 0, st>>>(e.rgb.as<float3>(), w, h, lum.as<float>(), rows.as<double>());
-    k_env_marginal<<<1, kEnvBlock, 0, st>>>(rows.as<double>(), h, mp.as<double>(), e.marginal.as<double>(),
+    FFTemp temp(ctx);
+    float* lum = temp.get<float>((size_t)w * h);
+    double* rows = temp.get<double>(h);
+    double* mp = temp.get<double>(h);
+    k_env_rows<<<h, kEnvBlock, 0, st>>>(e.rgb.as<float3>(), w, h, lum, rows);
+    k_env_marginal<<<1, kEnvBlock, 0, st>>>(rows, h, mp, e.marginal.as<double>(),
                                             e.denom.as<double>());
-    k_env_cond<<<h, kEnvBlock, 0, st>>>(lum.as<float>(), w, h, mp.as<double>(), e.denom.as<double>(),
+    k_env_cond<<<h, kEnvBlock, 0, st>>>(lum, w, h, mp, e.denom.as<double>(),
                                         e.conditional.as<double>(), e.pdf.as<float>());
     e.guide.alloc(sizeof(uint32_t) * ((size_t)kGuideMarginal + 1 + (size_t)h * (kGuideCond + 1)));
     k_env_guide<<<h + 1, kEnvBlock, 0, st>>>(e.marginal.as<double>(), e.conditional.as<double>(), w, h,

@@ -93,23 +93,25 @@ void ff_build_shading(ff_context* ctx, ff_scene* s, const ff_scene_desc* d, cons
 {
     cudaStream_t st = ctx->stream;
     const uint32_t n = d->num_triangles;
-    DevBuf nrm, uv, mat;
+    FFTemp temp(ctx);
+    float3* nrm = nullptr;
+    float2* uv = nullptr;
+    uint32_t* mat = nullptr;
     if (d->normals && d->num_vertices) {
-        nrm.alloc(sizeof(float3) * d->num_vertices);
-        FF_CUDA_CHECK(cudaMemcpyAsync(nrm.ptr, d->normals, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, st));
+        nrm = temp.get<float3>(d->num_vertices);
+        FF_CUDA_CHECK(cudaMemcpyAsync(nrm, d->normals, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, st));
     }
     if (d->texcoords && d->num_vertices) {
-        uv.alloc(sizeof(float2) * d->num_vertices);
-        FF_CUDA_CHECK(cudaMemcpyAsync(uv.ptr, d->texcoords, sizeof(float2) * d->num_vertices, cudaMemcpyHostToDevice, st));
+        uv = temp.get<float2>(d->num_vertices);
+        FF_CUDA_CHECK(cudaMemcpyAsync(uv, d->texcoords, sizeof(float2) * d->num_vertices, cudaMemcpyHostToDevice, st));
     }
     if (d->material_ids && n) {
-        mat.alloc(sizeof(uint32_t) * n);
-        FF_CUDA_CHECK(cudaMemcpyAsync(mat.ptr, d->material_ids, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
+        mat = temp.get<uint32_t>(n);
+        FF_CUDA_CHECK(cudaMemcpyAsync(mat, d->material_ids, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
     }
     if (n) {
         s->shade.alloc(sizeof(FFShadeTri) * n);
-        k_build_shading<<<(n + 255) / 256, 256, 0, st>>>(d_pos, d_idx, nrm.as<float3>(), uv.as<float2>(),
-                                                         mat.as<uint32_t>(), n, s->shade.as<FFShadeTri>());
+        k_build_shading<<<(n + 255) / 256, 256, 0, st>>>(d_pos, d_idx, nrm, uv, mat, n, s->shade.as<FFShadeTri>());
         FF_CUDA_CHECK(cudaGetLastError());
     }
     // Materials: a default grey FF_MAT_MIX when none are given.
@@ -136,20 +138,16 @@ void ff_build_shading(ff_context* ctx, ff_scene* s, const ff_scene_desc* d, cons
     FF_REQUIRE(!(d->tangents && !d->bitangents) && !(d->bitangents && !d->tangents),
                "tangents and bitangents come together");
     if (normal_maps && n) {
-        DevBuf tg, btg;
+        float3 *tg = nullptr, *btg = nullptr;
         if (d->tangents && d->num_vertices) {
-            tg.alloc(sizeof(float3) * d->num_vertices);
-            btg.alloc(sizeof(float3) * d->num_vertices);
-            FF_CUDA_CHECK(cudaMemcpyAsync(tg.ptr, d->tangents, sizeof(float3) * d->num_vertices,
-                                          cudaMemcpyHostToDevice, st));
-            FF_CUDA_CHECK(cudaMemcpyAsync(btg.ptr, d->bitangents, sizeof(float3) * d->num_vertices,
-                                          cudaMemcpyHostToDevice, st));
+            tg = temp.get<float3>(d->num_vertices);
+            btg = temp.get<float3>(d->num_vertices);
+            FF_CUDA_CHECK(cudaMemcpyAsync(tg, d->tangents, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, st));
+            FF_CUDA_CHECK(cudaMemcpyAsync(btg, d->bitangents, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, st));
         }
         s->tangent.alloc(sizeof(FFTangentTri) * n);
-        k_build_tangents<<<(n + 255) / 256, 256, 0, st>>>(d_pos, d_idx, uv.as<float2>(), tg.as<float3>(),
-                                                          btg.as<float3>(), n, s->tangent.as<FFTangentTri>());
+        k_build_tangents<<<(n + 255) / 256, 256, 0, st>>>(d_pos, d_idx, uv, tg, btg, n, s->tangent.as<FFTangentTri>());
         FF_CUDA_CHECK(cudaGetLastError());
-        FF_CUDA_CHECK(cudaStreamSynchronize(st));   // tg / btg are freed on return
     } else {
         s->tangent.release();
     }
@@ -164,9 +162,7 @@ void ff_build_shading(ff_context* ctx, ff_scene* s, const ff_scene_desc* d, cons
         for (uint32_t i = 0; i < d->num_textures; ++i) {
             const ff_texture_desc& td = d->textures[i];
             FF_REQUIRE(td.rgb && td.width > 0 && td.height > 0, "texture without texels");
-            DevBuf* b = new DevBuf();
-            s->textures.push_back(b);
-            b->alloc(sizeof(float3) * td.width * td.height);
+            DevBuf* b = s->textures[i];   // (placed at creation)
             FF_CUDA_CHECK(cudaMemcpyAsync(b->ptr, td.rgb, sizeof(float3) * td.width * td.height, cudaMemcpyHostToDevice, st));
             views[i] = FFTexView{b->as<float3>(), (int)td.width, (int)td.height};
         }

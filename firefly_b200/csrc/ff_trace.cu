@@ -444,10 +444,10 @@ void ff_launch_trace(ff_context* ctx, const ff_scene* s, const ff_ray* d_rays, u
 // Same launch as ff_launch_trace, with the work counter and the error counter
 // supplied by the caller instead of taken from the context's allocation.
 void ff_launch_trace_scratch(ff_context* ctx, const ff_scene* s, const ff_ray* d_rays, uint64_t n, ff_hit* d_hits,
-                             bool any_hit, unsigned long long* counter, unsigned int* err)
+                             bool any_hit, unsigned long long* counter, unsigned int* err, bool two_sided)
 {
     if (n == 0) return;
-    launch_trace(ctx, s->view(), d_rays, n, d_hits, any_hit, false, counter, err, nullptr, nullptr, nullptr, ctx->stream,
+    launch_trace(ctx, s->view(), d_rays, n, d_hits, any_hit, two_sided, counter, err, nullptr, nullptr, nullptr, ctx->stream,
                  0);
 }
 
