@@ -26,12 +26,9 @@ __device__ __forceinline__ Footprint footprint(int w, int h, float u, float v)
     ax = floorf(ax * 256.f + 0.5f) / 256.f;
     ay = floorf(ay * 256.f + 0.5f) / 256.f;
     int ix = (int)fx, iy = (int)fy;
-    int x0 = ix % w;
-    x0 = x0 < 0 ? x0 + w : x0;
-    int x1 = (x0 + 1 == w) ? 0 : x0 + 1;
-    int y0 = iy % h;
-    y0 = y0 < 0 ? y0 + h : y0;
-    int y1 = (y0 + 1 == h) ? 0 : y0 + 1;
+    const int x0 = wrap_index(ix, w), y0 = wrap_index(iy, h);
+    const int x1 = (x0 + 1 == w) ? 0 : x0 + 1;
+    const int y1 = (y0 + 1 == h) ? 0 : y0 + 1;
     Footprint f;
     f.idx[0] = y0 * w + x0;
     f.idx[1] = y0 * w + x1;

@@ -59,8 +59,24 @@ struct FFLightSet {
     bool corrected;
 };
 
+// What a kernel knows of the light when it is compiled: nothing, or that it is
+// the environment or an area light (one light for the whole launch), which
+// leaves the others' code and registers out.
+enum LightKind { LK_ANY = 0, LK_ENV = 1, LK_AREA = 2 };
+
+template <int KIND = LK_ANY>
 __device__ __forceinline__ LightCtx select_light(const FFLightSet& s, uint32_t key, uint32_t L)
 {
+    if (KIND != LK_ANY) {
+        LightCtx lc;
+        lc.env = s.env;
+        lc.corrected = s.corrected;
+        lc.is_env = KIND == LK_ENV;
+        lc.is_dir = false;
+        lc.scale = 1.f;
+        if (KIND == LK_AREA) lc.rect = make_rect(s.area[s.light]);
+        return lc;
+    }
     LightCtx lc;
     lc.env = s.env;
     lc.corrected = s.corrected;

@@ -514,6 +514,15 @@ FF_D float3 texel3(const float4* t, int i)
     const float4 v = t[i];
     return make_float3(v.x, v.y, v.z);
 }
+// Index i wrapped into [0, n).  (The remainder of a division by a run-time n
+// takes some 20 dependent instructions, and lookups lie within the texture
+// but for its border and repeated coordinates.)
+FF_D int wrap_index(int i, int n)
+{
+    if ((unsigned)i < (unsigned)n) return i;
+    i %= n;
+    return i < 0 ? i + n : i;
+}
 template <class T>
 FF_D float3 tex_bilinear(const T* texels, int w, int h, float u, float v)
 {
@@ -524,12 +533,9 @@ FF_D float3 tex_bilinear(const T* texels, int w, int h, float u, float v)
     ax = floorf(ax * 256.f + 0.5f) / 256.f;
     ay = floorf(ay * 256.f + 0.5f) / 256.f;
     int ix = (int)fx, iy = (int)fy;
-    int x0 = ix % w;
-    x0 = x0 < 0 ? x0 + w : x0;
-    int x1 = (x0 + 1 == w) ? 0 : x0 + 1;
-    int y0 = iy % h;
-    y0 = y0 < 0 ? y0 + h : y0;
-    int y1 = (y0 + 1 == h) ? 0 : y0 + 1;
+    const int x0 = wrap_index(ix, w), y0 = wrap_index(iy, h);
+    const int x1 = (x0 + 1 == w) ? 0 : x0 + 1;
+    const int y1 = (y0 + 1 == h) ? 0 : y0 + 1;
     float3 t00 = texel3(texels, y0 * w + x0), t10 = texel3(texels, y0 * w + x1);
     float3 t01 = texel3(texels, y1 * w + x0), t11 = texel3(texels, y1 * w + x1);
     float w00 = (1.f - ax) * (1.f - ay), w10 = ax * (1.f - ay), w01 = (1.f - ax) * ay, w11 = ax * ay;

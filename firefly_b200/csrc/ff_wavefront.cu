@@ -318,7 +318,7 @@ __device__ __forceinline__ bool path_ends(float3 f, float pdf)
 // current sample's radiance only, in plain FP32 adds as the megakernel
 // adjoint sums it; no film).
 constexpr int kLogicBlock = 256;
-template <bool ADJ>
+template <bool ADJ, int LK>
 __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                 if (!query) {
                     // Light sample (kernel.cu:435, light get_direction).
                     float3 wi, sp;
-                    sample_light(select_light(w.lights, key, L), pos, key, L, wi, sp);
+                    sample_light(select_light<LK>(w.lights, key, L), pos, key, L, wi, sp);
                     w.state[s] = PH_FLIGHT | L << kPhaseBits;
                     // (deferred mode: it still holds the throughput, unless the roulette scaled it)
                     if (ADJ || !w.defer || L > w.rr_depth) w.beta[s] = f4(beta);
@@ -682,7 +682,10 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
 // instantiation, which also leaves the vertex's derivative terms in the slot
 // during a replay.  CORR: corrected mode, whose reference lobes run in FP32
 // (parity mode keeps the reference's FP64 arithmetic; Lobes, ff_shade.cuh).
-template <int KIND, bool SEL, bool ADJ, bool CORR>
+// LK: what is known of the light (LightKind).  For the environment that
+// leaves 80 of the mix kind's 118 registers (6 instead of 4 blocks per SM),
+// for an area light 96.
+template <int KIND, bool SEL, bool ADJ, bool CORR, int LK>
 __global__ void __launch_bounds__(128) k_shade(WF w)
 {
     const uint32_t n = w.ctr[C_MAT + KIND];
@@ -695,7 +698,8 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
     uint32_t ext_base = w.ctr[C_CAM];
     for (int k = 0; k < KIND; ++k) ext_base += w.ctr[C_MAT + k];
     LightCtx lc;
-    if (!SEL) lc = select_light(w.lights, 0u, 0u);   // the fixed light
+    if (!SEL) lc = select_light<LK>(w.lights, 0u, 0u);   // the fixed light
+    lc.corrected = CORR;
     for (uint32_t it = 0; it < iters; ++it) {
         const uint32_t qi = base + it * stride;
         const bool valid = qi < n;
@@ -719,7 +723,10 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
             const float3 sp = make_float3(0.f, 0.f, 0.f);   // BRDF_L does not use the NEE sample point
             const uint32_t key = vx.key;
             const uint32_t L = (vx.word >> kVtxLenShift) & kVtxLenMask;
-            if (SEL) lc = select_light(w.lights, key, L);
+            if (SEL) {
+                lc = select_light(w.lights, key, L);
+                lc.corrected = CORR;
+            }
             o.c_spec = o.c_diff = make_float3(0.f, 0.f, 0.f);
             if (KIND == FF_MAT_MIX) shade_mix<CORR>(w.mode, lc, mat, pos, n, wo, wi, sp, key, L, o);
             else if (KIND == FF_MAT_DIFFUSE) shade_diffuse<CORR>(w.mode, lc, mat, pos, n, wo, wi, key, L, o);
@@ -947,10 +954,33 @@ T* carve(char*& p, size_t n)
     return r;
 }
 
+// What the launch knows of its light.
+LightKind light_kind(const WF& w)
+{
+    const int32_t light = w.lights.light;
+    if (light == -1) return LK_ENV;
+    return light >= 0 && (uint32_t)light < w.lights.n_area ? LK_AREA : LK_ANY;
+}
+
 template <int K, bool SEL, bool ADJ, bool CORR>
 void shade_kind(const WF& w, int blocks, cudaStream_t stream)
 {
-    k_shade<K, SEL, ADJ, CORR><<<blocks, 128, 0, stream>>>(w);
+    const LightKind lk = SEL ? LK_ANY : light_kind(w);
+    if constexpr (!SEL) {
+        if (lk == LK_ENV) k_shade<K, SEL, ADJ, CORR, LK_ENV><<<blocks, 128, 0, stream>>>(w);
+        if (lk == LK_AREA) k_shade<K, SEL, ADJ, CORR, LK_AREA><<<blocks, 128, 0, stream>>>(w);
+    }
+    if (lk == LK_ANY) k_shade<K, SEL, ADJ, CORR, LK_ANY><<<blocks, 128, 0, stream>>>(w);
+}
+
+template <bool ADJ>
+void launch_logic(const WF& w, cudaStream_t stream)
+{
+    const unsigned blocks = (w.P + kLogicBlock - 1) / kLogicBlock;
+    const LightKind lk = light_kind(w);
+    if (lk == LK_ENV) k_logic<ADJ, LK_ENV><<<blocks, kLogicBlock, 0, stream>>>(w);
+    else if (lk == LK_AREA) k_logic<ADJ, LK_AREA><<<blocks, kLogicBlock, 0, stream>>>(w);
+    else k_logic<ADJ, LK_ANY><<<blocks, kLogicBlock, 0, stream>>>(w);
 }
 
 // k_shade for every material kind in use.  With ws, the first kind runs on
@@ -1070,13 +1100,15 @@ void defer_setup(FFWavefrontWS* ws, uint32_t P, cudaStream_t stream)
 struct FrameLoop {
     FFWavefrontWS* ws;
     cudaStream_t stream;
+    int num_sms;
     uint32_t frames = 0;   // launched
     uint32_t cap;          // frames that always suffice
     uint32_t live;         // slots that can still have a ray, at most
     // `passes` passes over each sample; a sample takes at most max_depth + 1
     // frames a pass, the next one starts in the frame that ends it, and frame
     // 0 starts the first
-    FrameLoop(FFWavefrontWS* ws_, cudaStream_t stream_, const WF& w, uint32_t passes) : ws(ws_), stream(stream_)
+    FrameLoop(FFWavefrontWS* ws_, ff_context* ctx, const WF& w, uint32_t passes)
+        : ws(ws_), stream(ctx->stream), num_sms(ctx->num_sms)
     {
         live = ws->P;
         const uint64_t per_slot = (w.spp + w.m - 1) / w.m;
@@ -1117,6 +1149,12 @@ struct FrameLoop {
     // starts paths) and rays (every path has ended in the last possible one)
     bool has_vertices() const { return frames > 1 && has_rays(); }
     bool has_rays() const { return frames < cap; }
+    // Blocks of a k_shade launch: enough for every slot that can have a vertex,
+    // and at most 64 per SM, several times the 4 to 8 that are resident, so
+    // that the last ones end together (beside the any-hit trace they do not
+    // run alike).  ms per 64-spp step on the 1.3M-triangle scene with 6
+    // (resident) / 8 / 16 / 64 blocks per SM: 224.4 / 233.8 / 224.2 / 222.6.
+    int shade_blocks() const { return (int)std::min<uint64_t>((live + 127u) / 128u, (uint64_t)num_sms * 64u); }
     // Slots active after frame f, reported by k_logic of frame f + 1 (launched).
     uint32_t active_after(uint32_t f)
     {
@@ -1197,7 +1235,6 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
     w.defer = defer ? 1u : 0u;
     FF_CUDA_CHECK(cudaEventRecord(ctx->ev0, stream));
     if (defer) defer_setup(ws, P, stream);
-    int shade_blocks = ctx->num_sms * 8;
     int n_kinds = 0;
     for (int k = 0; k < kKinds; ++k) n_kinds += kind_used[k] ? 1 : 0;
     // Optional per-stage timing: events around the stages of every frame.
@@ -1211,7 +1248,7 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
         evs.push_back(e);
     };
     ws->ensure_streams();
-    FrameLoop loop(ws, stream, w, 1);
+    FrameLoop loop(ws, ctx, w, 1);
     uint32_t launches = 1;   // k_resolve
     // Deferred light terms (every render but the cached one): the any-hit
     // trace of frame f runs on the side stream beside k_logic, k_shade and
@@ -1229,7 +1266,7 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
         uint8_t* occ = defer ? reinterpret_cast<uint8_t*>(w.vis2 + (size_t)par * P) : reinterpret_cast<uint8_t*>(w.ray);
         if (defer && !profile && w.frame >= 2) FF_CUDA_CHECK(cudaStreamWaitEvent(stream, ws->sh_done[par], 0));
         mark();
-        k_logic<false><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
+        launch_logic<false>(w, stream);
         ++launches;
         mark();
         if (loop.has_vertices()) {
@@ -1237,9 +1274,9 @@ void ff_wavefront_render(ff_context* ctx, ff_scene* scene, const ff_render_setti
             FFWavefrontWS* side = profile ? nullptr : ws;
             const bool sel = w.lights.light == FF_LIGHT_ALL, corr = w.mode == FF_MODE_CORRECTED;
             // light selection needs the corrected mode (checked above)
-            if (sel) launch_shade<true, false, true>(w, kind_used, shade_blocks, stream, side);
-            else if (corr) launch_shade<false, false, true>(w, kind_used, shade_blocks, stream, side);
-            else launch_shade<false, false, false>(w, kind_used, shade_blocks, stream, side);
+            if (sel) launch_shade<true, false, true>(w, kind_used, loop.shade_blocks(), stream, side);
+            else if (corr) launch_shade<false, false, true>(w, kind_used, loop.shade_blocks(), stream, side);
+            else launch_shade<false, false, false>(w, kind_used, loop.shade_blocks(), stream, side);
             launches += (uint32_t)n_kinds;
         }
         FF_CUDA_CHECK(cudaGetLastError());
@@ -1460,7 +1497,6 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
     int n_kinds = 0;
     for (int k = 0; k < kKinds; ++k) n_kinds += kind_used[k] ? 1 : 0;
 
-    const int shade_blocks = ctx->num_sms * 8;
     // optional per-stage timing, as in ff_wavefront_render
     const bool profile = stats && (st->flags & FF_RENDER_PROFILE);
     std::vector<cudaEvent_t> evs;
@@ -1472,17 +1508,17 @@ void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_sett
         evs.push_back(e);
     };
     ws->ensure_streams();
-    FrameLoop loop(ws, stream, w, w.rec0 ? 1 : 2);
+    FrameLoop loop(ws, ctx, w, w.rec0 ? 1 : 2);
     uint32_t launches = 0;
     while (loop.next(w)) {
         unsigned long long* tctr = reinterpret_cast<unsigned long long*>(w.ctr + C_TRACE);
         mark();
-        k_logic<true><<<(P + kLogicBlock - 1) / kLogicBlock, kLogicBlock, 0, stream>>>(w);
+        launch_logic<true>(w, stream);
         ++launches;
         mark();
         // side streams as in ff_wavefront_render (one stream under stage timing)
         if (loop.has_vertices()) {
-            launch_shade<false, true, true>(w, kind_used, shade_blocks, stream, profile ? nullptr : ws);
+            launch_shade<false, true, true>(w, kind_used, loop.shade_blocks(), stream, profile ? nullptr : ws);
             launches += (uint32_t)n_kinds;
         }
         FF_CUDA_CHECK(cudaGetLastError());
