@@ -133,6 +133,42 @@ struct __align__(16) FFTri {
 // (FFRayState::prim, and the material word of a path vertex).
 constexpr uint32_t kBackFace = 0x80000000u;
 
+#ifdef __CUDACC__
+// A 32-byte record (on a 32-byte boundary) in one access.  Two 16-byte stores
+// of neighbouring lanes' records each touch every other half sector, so L2
+// takes twice the writes; the loads' second half is a second pass over the
+// same lines.  With every per-slot and queue record moved so, the
+// 1.3M-triangle 64-spp step went from 220.6 to 204.5 ms, the inverse step from
+// 10.4 to 9.6 ms, the small room from 2.11 to 2.07 ms.
+template <class T>
+__device__ __forceinline__ T ld_sector(const T* p)
+{
+    static_assert(sizeof(T) == 32, "one sector");
+    union {
+        uint32_t u[8];
+        T v;
+    } r;
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r.u[0]), "=r"(r.u[1]), "=r"(r.u[2]), "=r"(r.u[3]), "=r"(r.u[4]), "=r"(r.u[5]), "=r"(r.u[6]),
+                   "=r"(r.u[7])
+                 : "l"(p));
+    return r.v;
+}
+template <class T>
+__device__ __forceinline__ void st_sector(T* p, const T& v)
+{
+    static_assert(sizeof(T) == 32, "one sector");
+    union U {
+        uint32_t u[8];
+        T v;
+        __device__ U(const T& t) : v(t) {}
+    } r(v);
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r.u[0]), "r"(r.u[1]),
+                 "r"(r.u[2]), "r"(r.u[3]), "r"(r.u[4]), "r"(r.u[5]), "r"(r.u[6]), "r"(r.u[7])
+                 : "memory");
+}
+#endif
+
 struct FFBvhView {
     const FFNode8* nodes;
     const FFTri* tris;

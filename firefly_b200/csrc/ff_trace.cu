@@ -67,9 +67,16 @@ __global__ void __launch_bounds__(kTraceBlock, 8)
             if (!active && !exhausted) {
                 ray_id = base + __popc(want & lt_mask);
                 if (ray_id < n) {
-                    const float4 r0 = __ldg(reinterpret_cast<const float4*>(rays + ray_id));
-                    const float4 r1 = __ldg(reinterpret_cast<const float4*>(rays + ray_id) + 1);
-                    if (TAGGED) tag = __ldg(tags + ray_id);
+                    float4 r0, r1;
+                    if (TAGGED) {   // (a queue's rays sit on 32-byte boundaries, a caller's on 16)
+                        const ff_ray q = ld_sector(rays + ray_id);
+                        r0 = make_float4(q.ox, q.oy, q.oz, q.tmin);
+                        r1 = make_float4(q.dx, q.dy, q.dz, q.tmax);
+                        tag = __ldg(tags + ray_id);
+                    } else {
+                        r0 = __ldg(reinterpret_cast<const float4*>(rays + ray_id));
+                        r1 = __ldg(reinterpret_cast<const float4*>(rays + ray_id) + 1);
+                    }
                     // untagged two-sided launches (ff_trace with FF_TRACE_TWO_SIDED) mark every ray;
                     // tagged ones (the wavefront) carry the mark in each ray's tmin
                     const float tmin = (TWO && !TAGGED) ? -(r0.w > 0.f ? r0.w : 0.f) : r0.w;

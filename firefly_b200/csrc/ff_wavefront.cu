@@ -93,28 +93,36 @@ struct __align__(32) SlotMis {
 };
 // The vertex k_logic hands to k_shade.  word = material index (bits 0-23) |
 // path length (bits 24-30) | hit from inside an object (bit 31).
-struct __align__(32) SlotVtx {
+struct __align__(32) SlotVtxA {
     float px, py, pz;
     uint32_t word;
     float nx, ny, nz;   // shading normal
     uint32_t key;
+};
+struct __align__(32) SlotVtxB {
     float wix, wiy, wiz;   // NEE direction
     float u;
     float wox, woy, woz;   // toward the previous vertex
     float v;
+};
+struct SlotVtx {
+    SlotVtxA a;
+    SlotVtxB b;
 };
 // Deferred light terms (ff_render without the cache): what a vertex's
 // shading leaves for the k_logic two frames later, after the any-hit trace
 // that runs beside the next frame has answered its shadow rays: the
 // throughput at the vertex, the frame stamp, the three light terms and the
 // rays queued.  Indexed [frame parity][slot].
-struct __align__(32) SlotPend {
+struct __align__(32) SlotPendA {
     float bx, by, bz;
     uint32_t stamp;   // WF::stamp0 + frame of the shading; any other value: nothing pending
     float nee_x, nee_y, nee_z;
     uint32_t queued;  // bit k: shadow ray k was queued
-    float spec_x, spec_y, spec_z, pad0;
-    float diff_x, diff_y, diff_z, pad1;
+};
+struct SlotPend {
+    SlotPendA a;
+    SlotMis b;   // the BSDF-sampled light terms
 };
 static_assert(sizeof(SlotRay) == 32 && sizeof(SlotShade) == 32 && sizeof(SlotMis) == 32 && sizeof(SlotVtx) == 64 &&
                   sizeof(SlotPend) == 64,
@@ -270,7 +278,7 @@ __device__ __forceinline__ void start_sample(const WF& w, uint32_t s, uint32_t s
     const int x = (int)(pix % w.W), y = (int)(pix / w.W);
     float3 o, d;
     gen_camera_ray(w.cam, (int)w.W, (int)w.H, x, y, rand2(key, 0, DIM_CAM_JITTER), rand2(key, 0, DIM_CAM_LENS), o, d);
-    w.ray[s] = SlotRay{o.x, o.y, o.z, 0u, d.x, d.y, d.z, 0.f};
+    st_sector(w.ray + s, SlotRay{o.x, o.y, o.z, 0u, d.x, d.y, d.z, 0.f});
     ray = ff_ray{o.x, o.y, o.z, 0.f, d.x, d.y, d.z, __int_as_float(0x7f800000)};
 }
 
@@ -282,29 +290,23 @@ __device__ __forceinline__ void start_sample(const WF& w, uint32_t s, uint32_t s
 __device__ __forceinline__ bool consume_pending(const WF& w, uint32_t frame, uint32_t s, float4& acc, float4& accc)
 {
     const size_t i = (size_t)(frame & 1u) * w.P + s;
-    const float4* pq = reinterpret_cast<const float4*>(w.pend + i);
-    const float4 a = pq[0];
-    if (__float_as_uint(a.w) != w.stamp0 + frame - 2u) return false;
-    const float4 b = pq[1];
-    const uint32_t q = __float_as_uint(b.w);
+    const SlotPendA p = ld_sector(&w.pend[i].a);
+    if (p.stamp != w.stamp0 + frame - 2u) return false;
+    const uint32_t q = p.queued;
     const uint32_t vw = w.vis2[i];
     const bool vis = (q & 1u) && !(vw & 0xffu);
     const bool vis_s = (q & 2u) && !(vw & 0xff00u);
     const bool vis_d = (q & 4u) && !(vw & 0xff0000u);
-    const float3 beta = xyz(a);
-    if (w.mode == FF_MODE_CORRECTED) {
-        float3 lb = make_float3(0.f, 0.f, 0.f);
-        if (vis) lb = lb + xyz(b);
-        if (vis_s) lb = lb + xyz(pq[2]);
-        if (vis_d) lb = lb + xyz(pq[3]);
-        if (vis || vis_s || vis_d) kahan_add(acc, accc, lb * beta);
-    } else if (vis) {
-        // parity: the whole light_brdf, MIS terms included, rides on the NEE ray
-        float3 lb = xyz(b);
-        if (vis_s) lb = lb + xyz(pq[2]);
-        if (vis_d) lb = lb + xyz(pq[3]);
-        kahan_add(acc, accc, lb * beta);
+    // parity: the whole light_brdf, MIS terms included, rides on the NEE ray
+    if (!(w.mode == FF_MODE_CORRECTED ? vis || vis_s || vis_d : vis)) return true;
+    float3 lb = make_float3(0.f, 0.f, 0.f);
+    if (vis) lb = lb + make_float3(p.nee_x, p.nee_y, p.nee_z);
+    if (vis_s || vis_d) {
+        const SlotMis m = ld_sector(&w.pend[i].b);
+        if (vis_s) lb = lb + make_float3(m.spec_x, m.spec_y, m.spec_z);
+        if (vis_d) lb = lb + make_float3(m.diff_x, m.diff_y, m.diff_z);
     }
+    kahan_add(acc, accc, lb * make_float3(p.bx, p.by, p.bz));
     return true;
 }
 
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
             const ff_hit hit = w.ext_hits[s];
             const uint32_t L = (state >> kPhaseBits) + 1;  // wf_extend's length++
             const bool found = hit.prim != -1;
-            const SlotRay sr = w.ray[s];
+            const SlotRay sr = ld_sector(w.ray + s);
             const float3 ro = make_float3(sr.ox, sr.oy, sr.oz), rd = make_float3(sr.dx, sr.dy, sr.dz);
             const float4 beta4 = w.beta[s];
             float3 beta = xyz(beta4);
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                     // light terms were added above; k_shade left the throughput after the vertex
                     ends = beta4.w != 0.f;
                 } else {
-                    const SlotShade sd = w.shd[s];
+                    const SlotShade sd = ld_sector(w.shd + s);
                     // kernel.cu:357-359: light_brdf * beta when the NEE ray was unoccluded
                     const uint32_t vw = sr.vis;
                     const bool vis = (vw & (1u << 24)) && !(vw & 0xffu);
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                         float3 lb = make_float3(0.f, 0.f, 0.f);
                         if (vis) lb = lb + make_float3(sd.nee_x, sd.nee_y, sd.nee_z);
                         if (vis_s || vis_d) {
-                            const SlotMis sm = w.mis[s];
+                            const SlotMis sm = ld_sector(w.mis + s);
                             if (vis_s) lb = lb + make_float3(sm.spec_x, sm.spec_y, sm.spec_z);
                             if (vis_d) lb = lb + make_float3(sm.diff_x, sm.diff_y, sm.diff_z);
                         }
@@ -426,7 +428,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                                 // the previous vertex's gradients, now that its shadow rays are answered
                                 const float4 va = w.v_albedo[s];
                                 const uint32_t flags = __float_as_uint(va.w);
-                                const SlotVtx& pv = w.vtx[s];   // the previous vertex
+                                const SlotVtxB pv = ld_sector(&w.vtx[s].b);   // the previous vertex
                                 const float2 uv = make_float2(pv.u, pv.v);
                                 if (record && (flags & (V_ALBEDO | V_ROUGH))) {
                                     const size_t i = (size_t)kept * w.P + s;
@@ -482,7 +484,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                         // parity: the whole light_brdf, MIS terms included, rides on the NEE ray
                         float3 lb = make_float3(sd.nee_x, sd.nee_y, sd.nee_z);
                         if (vis_s || vis_d) {
-                            const SlotMis sm = w.mis[s];
+                            const SlotMis sm = ld_sector(w.mis + s);
                             if (vis_s) lb = lb + make_float3(sm.spec_x, sm.spec_y, sm.spec_z);
                             if (vis_d) lb = lb + make_float3(sm.diff_x, sm.diff_y, sm.diff_z);
                         }
@@ -546,16 +548,18 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
                     w.state[s] = PH_FLIGHT | L << kPhaseBits;
                     // (deferred mode: it still holds the throughput, unless the roulette scaled it)
                     if (ADJ || !w.defer || L > w.rr_depth) w.beta[s] = f4(beta);
-                    SlotVtx vx;
+                    SlotVtxA vx;
+                    SlotVtxB vy;
                     vx.px = pos.x, vx.py = pos.y, vx.pz = pos.z;
                     vx.word = t.material | (L << kVtxLenShift) | (back ? kBackFace : 0u);
                     vx.nx = ns.x, vx.ny = ns.y, vx.nz = ns.z;
                     vx.key = key;
-                    vx.wix = wi.x, vx.wiy = wi.y, vx.wiz = wi.z;   // (the sample point is not needed downstream)
-                    vx.u = uv.x;
-                    vx.wox = -rd.x, vx.woy = -rd.y, vx.woz = -rd.z;
-                    vx.v = uv.y;
-                    w.vtx[s] = vx;
+                    vy.wix = wi.x, vy.wiy = wi.y, vy.wiz = wi.z;   // (the sample point is not needed downstream)
+                    vy.u = uv.x;
+                    vy.wox = -rd.x, vy.woy = -rd.y, vy.woz = -rd.z;
+                    vy.v = uv.y;
+                    st_sector(&w.vtx[s].a, vx);
+                    st_sector(&w.vtx[s].b, vy);
                     if (mm.normal_tex >= 0) w.hit_ngeo[s] = f4(n);
                     kind = mm.kind;
                 }
@@ -663,7 +667,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
         if (kind >= 0) {
             w.mat_queue[(size_t)kind * w.P + pos] = s;
         } else {
-            w.ext_rays[pos] = ray;
+            st_sector(w.ext_rays + pos, ray);
             w.ext_tag[pos] = s;
         }
     }
@@ -709,17 +713,18 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
         uint32_t s = 0;
         if (valid) {
             s = w.mat_queue[(size_t)KIND * w.P + qi];
-            const SlotVtx vx = w.vtx[s];
+            const SlotVtxA vx = ld_sector(&w.vtx[s].a);
+            const SlotVtxB vy = ld_sector(&w.vtx[s].b);
             const float3 pos = make_float3(vx.px, vx.py, vx.pz);
             const bool back = (vx.word & kBackFace) != 0;   // hit from inside an object
             const ff_material& mm = w.mats[vx.word & ((1u << kVtxMatBits) - 1u)];
-            const FFSurf mat = resolve_surface(mm, w.tex, make_float2(vx.u, vx.v));
+            const FFSurf mat = resolve_surface(mm, w.tex, make_float2(vy.u, vy.v));
             const float3 n = make_float3(vx.nx, vx.ny, vx.nz);   // shading normal
             // the normal the ray offsets follow (kernel.cu:437): differs from n
             // only under a normal texture
             const float3 ng = mm.normal_tex >= 0 ? xyz(w.hit_ngeo[s]) : n;
-            const float3 wo = make_float3(vx.wox, vx.woy, vx.woz);
-            const float3 wi = make_float3(vx.wix, vx.wiy, vx.wiz);
+            const float3 wo = make_float3(vy.wox, vy.woy, vy.woz);
+            const float3 wi = make_float3(vy.wix, vy.wiy, vy.wiz);
             const float3 sp = make_float3(0.f, 0.f, 0.f);   // BRDF_L does not use the NEE sample point
             const uint32_t key = vx.key;
             const uint32_t L = (vx.word >> kVtxLenShift) & kVtxLenMask;
@@ -747,10 +752,12 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
                 o.ext_o = pos + ng * (side * w.shadow_offset);
             ext_two = runs_inside(back, KIND == FF_MAT_DIELECTRIC, side);
             if (ADJ || !w.defer)
-                w.shd[s] = SlotShade{o.c_nee.x, o.c_nee.y, o.c_nee.z, o.ext_pdf, o.ext_f.x, o.ext_f.y, o.ext_f.z, o.ext_cos};
+                st_sector(w.shd + s, SlotShade{o.c_nee.x, o.c_nee.y, o.c_nee.z, o.ext_pdf, o.ext_f.x, o.ext_f.y, o.ext_f.z,
+                                               o.ext_cos});
             // the kinds with BSDF-sampled light terms (deferred mode: in the pending record)
             if ((KIND == FF_MAT_MIX || KIND == FF_MAT_DIELECTRIC) && (ADJ || !w.defer))
-                w.mis[s] = SlotMis{o.c_spec.x, o.c_spec.y, o.c_spec.z, 0.f, o.c_diff.x, o.c_diff.y, o.c_diff.z, 0.f};
+                st_sector(w.mis + s,
+                          SlotMis{o.c_spec.x, o.c_spec.y, o.c_spec.z, 0.f, o.c_diff.x, o.c_diff.y, o.c_diff.z, 0.f});
             if (ADJ && (w.rec0 || w.pass[s] != 0u)) {
                 uint32_t flags = 0;
                 if (KIND == FF_MAT_DIFFUSE && w.grad_tex && mm.base_color_tex >= 0 && mm.base_color_tex == w.adj_texture)
@@ -786,19 +793,21 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
         const bool defer = !ADJ && w.defer;
         if (valid) {
             const uint32_t qe = ext_base + qi;
-            w.ext_rays[qe] = make_ext_ray(o.ext_o, o.ext_d, ext_two);
+            st_sector(w.ext_rays + qe, make_ext_ray(o.ext_o, o.ext_d, ext_two));
             w.ext_tag[qe] = s;
             // the continuation ray and the queued-rays byte, one whole record
             const uint32_t queued = ((o.ray_nee ? 1u : 0u) | (o.ray_spec ? 2u : 0u) | (o.ray_diff ? 4u : 0u)) << 24;
-            w.ray[s] = SlotRay{o.ext_o.x, o.ext_o.y, o.ext_o.z, queued, o.ext_d.x, o.ext_d.y, o.ext_d.z, 0.f};
+            st_sector(w.ray + s, SlotRay{o.ext_o.x, o.ext_o.y, o.ext_o.z, queued, o.ext_d.x, o.ext_d.y, o.ext_d.z, 0.f});
             if (defer) {
                 // the light terms with the throughput they multiply, for k_logic two frames on
                 const float4 beta_v = w.beta[s];   // the throughput at this vertex
-                float4* pq = reinterpret_cast<float4*>(w.pend + (size_t)w.par * w.P + s);
-                pq[0] = make_float4(beta_v.x, beta_v.y, beta_v.z, __uint_as_float(w.stamp0 + w.frame));
-                pq[1] = make_float4(o.c_nee.x, o.c_nee.y, o.c_nee.z, __uint_as_float(queued >> 24));
-                pq[2] = f4(o.c_spec);
-                pq[3] = f4(o.c_diff);
+                SlotPend* pq = w.pend + (size_t)w.par * w.P + s;
+                st_sector(&pq->a, SlotPendA{beta_v.x, beta_v.y, beta_v.z, w.stamp0 + w.frame, o.c_nee.x, o.c_nee.y,
+                                            o.c_nee.z, queued >> 24});
+                // (read only where one of its rays was queued)
+                if (queued & (6u << 24))
+                    st_sector(&pq->b,
+                              SlotMis{o.c_spec.x, o.c_spec.y, o.c_spec.z, 0.f, o.c_diff.x, o.c_diff.y, o.c_diff.z, 0.f});
                 // and the throughput after it in the place of the one before: 16
                 // bytes of a sector just read, where its factors took a record of
                 // 32 here and 32 more to read in k_logic.  With that, the sample
@@ -817,15 +826,15 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
         const uint32_t q0 = sh_base + __popc(m0 & below), q1 = sh_base + n0 + __popc(m1 & below),
                        q2 = sh_base + n0 + n1 + __popc(m2 & below);
         if (o.ray_nee) {
-            w.sh_rays[q0] = o.r_nee;
+            st_sector(w.sh_rays + q0, o.r_nee);
             w.sh_tag[q0] = defer ? 4u * s : vis_byte(s, 0);
         }
         if (o.ray_spec) {
-            w.sh_rays[q1] = o.r_spec;
+            st_sector(w.sh_rays + q1, o.r_spec);
             w.sh_tag[q1] = defer ? 4u * s + 1u : vis_byte(s, 1);
         }
         if (o.ray_diff) {
-            w.sh_rays[q2] = o.r_diff;
+            st_sector(w.sh_rays + q2, o.r_diff);
             w.sh_tag[q2] = defer ? 4u * s + 2u : vis_byte(s, 2);
         }
     }
