@@ -19,6 +19,8 @@ constexpr int kTraceBlock = 128;
 // Refill when at least this many lanes of the warp are idle.
 constexpr int kRefillIdle = 8;
 
+constexpr uint32_t kPool = 64;
+
 // Output: hits[ray] for every ray, or, with tags (the wavefront's queues),
 // per the ray's tag: a closest hit goes to hits[tag] (tag = the path slot, so
 // the next stage reads its hit in slot order without the queue index), an
@@ -55,17 +57,37 @@ __global__ void __launch_bounds__(kTraceBlock, 8)
     uint32_t steps = 0;
     bool active = false;
     bool exhausted = false;
+    // the warp's share of the rays: pool_left of them from pool_next.  A
+    // caller's rays are taken kPool at a time (all warps' atomics go to one
+    // address, one after the other), near the end only as many as needed, so
+    // that the last ones spread over all warps: 16.8M incoherent closest hits
+    // 1419 -> 1381 us, 3M any hits 231 -> 226 us.  The wavefront's queues are
+    // short, and their tails weigh more (256 x 256 x 16 render 2.06 -> 2.09
+    // ms): there a warp takes what its idle lanes need.
+    uint64_t pool_next = 0;
+    uint32_t pool_left = 0;
 
     while (true) {
         // Refill idle lanes with new rays.
         const uint32_t want = __ballot_sync(0xffffffffu, !active && !exhausted);
         if (want) {
-            const uint32_t leader = __ffs(want) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(want));
-            base = __shfl_sync(0xffffffffu, base, leader);
+            const uint32_t need = __popc(want), rank = __popc(want & lt_mask);
+            uint64_t mine = pool_next + rank;
+            if (pool_left < need) {
+                const uint32_t more = need - pool_left;
+                const uint32_t take = !TAGGED && pool_next + (uint64_t)gridDim.x * (2u * kTraceBlock) < n ? kPool : more;
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(counter, (unsigned long long)take);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (rank >= pool_left) mine = base + (rank - pool_left);
+                pool_next = base + more;
+                pool_left = take - more;
+            } else {
+                pool_next += need;
+                pool_left -= need;
+            }
             if (!active && !exhausted) {
-                ray_id = base + __popc(want & lt_mask);
+                ray_id = mine;
                 if (ray_id < n) {
                     float4 r0, r1;
                     if (TAGGED) {   // (a queue's rays sit on 32-byte boundaries, a caller's on 16)
