@@ -49,6 +49,30 @@ struct alignas(16) Record {
 };
 static_assert(sizeof(Record) == 64, "record layout");
 
+// A record in two 32-byte accesses; the loads only where the array sits on a
+// 32-byte boundary (a caller's may not).
+struct __align__(32) RecordHalf {
+    float f[8];
+};
+__device__ __forceinline__ void store_record(Record* p, const Record& r)
+{
+    const RecordHalf* h = reinterpret_cast<const RecordHalf*>(&r);
+    RecordHalf* q = reinterpret_cast<RecordHalf*>(p);
+    st_sector(q, h[0]);
+    st_sector(q + 1, h[1]);
+}
+__device__ __forceinline__ Record load_record(const Record* p)
+{
+    if (reinterpret_cast<uintptr_t>(p) & 31u) return *p;
+    union {
+        RecordHalf h[2];
+        Record r;
+    } u;
+    u.h[0] = ld_sector(reinterpret_cast<const RecordHalf*>(p));
+    u.h[1] = ld_sector(reinterpret_cast<const RecordHalf*>(p) + 1);
+    return u.r;
+}
+
 __device__ __forceinline__ Record make_record(float3 pos, float rough, float3 wo, float3 n, float3 v, uint32_t pixel)
 {
     Record r;

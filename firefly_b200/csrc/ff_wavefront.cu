@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
             }
             if (!ADJ && w.cache_mode) {
                 const uint32_t qi = warp_append(w.n_queries, query);
-                if (query) w.queries[qi] = rec;
+                if (query) store_record(w.queries + qi, rec);
             }
         } else if (!ADJ && w.defer && ph == PH_DONE) {
             // a slot that finished in the previous frame: the light terms of its
