@@ -22,7 +22,7 @@ format as its own --workload line):
                   ff_trace), with the reference's own GPU traversal on the same
                   rays and every ray checked against the oracle;
   small_room      the plain tracer on the small room, 256 x 256 x 16 spp;
-  adjoint         path-replay adjoint samples per second (inverse rendering);
+  adjoint         adjoint samples per second (inverse rendering);
   radiance_cache  time to relMSE 0.01 with the learned radiance cache against
                   the plain tracer.
 --render-only skips them.
@@ -60,36 +60,35 @@ NODE_BYTES, TRI_BYTES = 80, 48
 # The wavefront's traces read a tagged queue (32 B ray + 4 B tag): the
 # closest-hit trace writes a 16 B hit, the any-hit trace a 1 B answer.
 WF_CLOSEST_BYTES, WF_ANY_BYTES = 32 + 4 + 16, 32 + 4 + 1
-# k_logic in the adjoint, per slot in flight and frame (continuing path):
-# reads phase, key, ext_q, length, pass (20 B), the extension hit (16), ray
-# origin and direction (32), throughput (16), radiance sum (16), shadow-queue
-# indices (16) and ~1.5 shadow hits (24), the three light terms (48), ext_f /
-# pdf / cos (20), the triangle's shading record (64); writes the sum (16) and
-# the next vertex (uv, length, throughput, position, normal, light sample,
-# queue entry: 112).  The replay pass adds dL/dI (12), L_s (16) and the
-# vertex record (albedo + flags, uv, env coefficient, light direction: 56).
-# Primal ~398 B, replay ~478 B: 438 B on average.
-ADJ_LOGIC_BYTES_PER_HIT = 438
+# k_logic in the adjoint, per consumed extension hit: reads the slot words
+# (12 B), the hit (16), the ray record (32), throughput (16), sum and
+# compensation (32), the shading and light-term records (64), the triangle's
+# shading attributes (64), the vertex's derivative terms (albedo + flags, uv,
+# env coefficient, light direction: 56) and, once the sample ends, its vertex
+# record (32); writes sum, compensation, throughput and state (52), the next
+# vertex (64) and the vertex record (32): 472 B.  Every path is traced once;
+# the reported rays count it twice, as an adjoint that replays does.
+ADJ_LOGIC_BYTES_PER_HIT = 472
+ADJ_PASSES_REPORTED = 2
 # k_logic in ff_render, per consumed extension hit of a continuing path:
-# reads the slot words (12 B), the hit (16), the ray record (32), throughput,
-# sum and compensation (48), the shading record (32), the pending light-term
-# record of two frames back and its answer word (68) and the triangle's
-# shading attributes (64); writes sum, compensation, length and throughput
-# (52) and the vertex record (64): 388 B.
-RENDER_LOGIC_BYTES_PER_HIT = 388
+# reads the slot words (8 B), the hit (16), the ray record (32), throughput,
+# sum and compensation (48), the pending light-term record of two frames back
+# and its answer word (68) and the triangle's shading attributes (64); writes
+# sum, compensation and state (36) and the vertex record (64): 336 B.
+RENDER_LOGIC_BYTES_PER_HIT = 336
 # k_shade, per shaded vertex: reads the vertex record (64 B), its queue
-# entry (4) and the throughput (16), writes the shading record (32), the ray
+# entry (4) and the throughput (16), writes the throughput (16), the ray
 # record (32), the extension-queue entry (36) and the pending light-term
-# record (64): 248 B; plus 36 B per shadow-queue entry (32 B ray, 4 B tag).
+# record (64): 232 B; plus 36 B per shadow-queue entry (32 B ray, 4 B tag).
 # Environment and material lookups are L2 gathers and not counted.
-RENDER_SHADE_BYTES_PER_VERTEX = 248
+RENDER_SHADE_BYTES_PER_VERTEX = 232
 SHADOW_QUEUE_BYTES = 36
 # Measured DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unit
 # of each render stage: ncu over every launch of one timed 16-spp C2 step on
-# a 2,097,152-slot pool (104 frames), divided by the step's units (consumed
+# a 2,097,152-slot pool (102 frames), divided by the step's units (consumed
 # hits, shaded vertices, extension rays, shadow rays).
-RENDER_DRAM_BYTES_PER_UNIT = {"k_logic": 456.8, "k_shade (all kinds)": 418.7,
-                              "k_trace<closest> (extension queue)": 109.4, "k_trace<any> (shadow queue)": 48.5}
+RENDER_DRAM_BYTES_PER_UNIT = {"k_logic": 343.3, "k_shade (all kinds)": 408.0,
+                              "k_trace<closest> (extension queue)": 107.5, "k_trace<any> (shadow queue)": 48.4}
 # Issue slots busy (smsp__issue_active) of the closest-hit traversal on C2:
 # ncu --set full of one steady-state launch of the same 16-spp, 2M-slot step
 # (a figure from that capture, not measured by this run).
@@ -954,7 +953,7 @@ def small_room_line(args, ws, rank, local, dist, ctx, dev, stream, steps=20, war
 
 INVERSE_WORKLOAD = ("inverse rendering on the room opened to the sky at 512x512: hidden 512x512 Perlin albedo in "
                     "[0.1, 0.9] + 256x128 hazy sky (sun radiance 8, 20 deg); target at 256 spp; start 0.5 albedo + "
-                    "flat env; 16-spp path-replay adjoint, Adam lr 1e-2 falling geometrically to 1e-3, 200 steps")
+                    "flat env; 16-spp adjoint, Adam lr 1e-2 falling geometrically to 1e-3, 200 steps")
 
 
 def inverse_experiment(ctx, steps=200, res=512, dev=None, known_lighting=False, rank=0, world=1):
@@ -1052,14 +1051,16 @@ def inverse_line(args, ws, rank, local, dist, ctx, dev, stream, known_lighting_r
                   "k_trace any (shadow)": prof["ms_trace_shadow"]}
         r["adjoint_stage_ms"] = {k: round(v, 3) for k, v in stages.items()}
         r["adjoint_rays"] = {"extension": prof["extension_rays"], "shadow": prof["shadow_rays"]}
+        ext_traced = prof["extension_rays"] // ADJ_PASSES_REPORTED
+        shadow_traced = prof["shadow_rays"] // ADJ_PASSES_REPORTED
         dom = max(stages, key=stages.get)
         if dom.startswith("k_logic"):
             # one consumed extension hit per slot and frame
-            achieved = prof["extension_rays"] * ADJ_LOGIC_BYTES_PER_HIT / (stages[dom] / 1e3) / 1e9
-            note = (f"algorithmic bytes = {ADJ_LOGIC_BYTES_PER_HIT} B of slot state read and written per consumed "
-                    "extension hit (primal and replay passes averaged) over the stage's event-timed duration")
+            achieved = ext_traced * ADJ_LOGIC_BYTES_PER_HIT / (stages[dom] / 1e3) / 1e9
+            note = (f"algorithmic bytes = {ADJ_LOGIC_BYTES_PER_HIT} B of slot state and records read and written per "
+                    "consumed extension hit over the stage's event-timed duration")
         elif "trace" in dom:
-            rays = prof["extension_rays"] if "closest" in dom else prof["shadow_rays"]
+            rays = ext_traced if "closest" in dom else shadow_traced
             per = WF_CLOSEST_BYTES if "closest" in dom else WF_ANY_BYTES
             achieved = rays * per / (stages[dom] / 1e3) / 1e9
             note = (f"algorithmic bytes = {per} B per ray (32 B ray + 4 B tag in, the hit or answer out) x the "
@@ -1071,8 +1072,8 @@ def inverse_line(args, ws, rank, local, dist, ctx, dev, stream, known_lighting_r
                     "(counted by the kernels) over the whole adjoint")
         # DRAM traffic of the dominant stage per frame: measured bytes per
         # unit (ncu over the profiled call) x this call's units per frame
-        units = {"k_logic (adjoint)": prof["extension_rays"], "k_shade (adjoint)": prof["extension_rays"],
-                 "k_trace closest (extension)": prof["extension_rays"], "k_trace any (shadow)": prof["shadow_rays"]}
+        units = {"k_logic (adjoint)": ext_traced, "k_shade (adjoint)": ext_traced,
+                 "k_trace closest (extension)": ext_traced, "k_trace any (shadow)": shadow_traced}
         traffic = int(ADJ_DRAM_BYTES_PER_UNIT[dom] * units[dom] / max(1, prof["frames"]))
         cpu = None if args.no_cpu else inverse_cpu_baseline(target_s=args.cpu_s)
         line = {"metric": "adjoint spp/s", "value": round(value, 1), "unit": "samples/s", "n_gpus": ws,
