@@ -11,7 +11,8 @@
 //      of the cheapest collapse of every subtree              (k_bounds_up)
 //   6. top-down collapse into 8-wide nodes along the plan,
 //      octant-ordered slots, 8-bit conservative quantisation,
-//      leaves of up to 3 consecutive triangles                (k_collapse, one launch per level)
+//      leaves of up to 3 consecutive triangles                (k_collapse, one launch per level,
+//      four between looks of the host)
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -366,15 +367,29 @@ FF_D int quant_exp(float lo, float hi)
     return e;
 }
 
-__global__ void k_collapse(const CollapseItem* __restrict__ in, uint32_t n_in, CollapseItem* __restrict__ out,
-                           uint32_t* __restrict__ counters /* 0: out size, 1: node count, 2: tri count, 3: error */,
+constexpr int kCollapseBlock = 32;
+constexpr int kLevelsAhead = 4;
+constexpr int kMaxLevels = 200;   // (a multiple of kLevelsAhead)
+static_assert(kMaxLevels % kLevelsAhead == 0);
+
+// One level of the collapse, one thread a wide node: a serial chain (the
+// planned subtree, the swaps, the quantisation) of about 25 us whatever the
+// level's size, so blocks of one warp spread a level over the SMs.  The
+// level's size is read here, not on the host: several levels are launched
+// between two looks of the host, over the most nodes each can have.  Loading
+// 82k triangles 2,280 us with a look a level and blocks of 128, 2,080 so;
+// 1,300 triangles 1,650 and 1,530; eight levels between looks 2,085 to 2,160.
+__global__ void __launch_bounds__(kCollapseBlock)
+    k_collapse(const CollapseItem* __restrict__ in, CollapseItem* __restrict__ out,
+                           uint32_t* __restrict__ level /* this level's items, then the next one's */,
+                           uint32_t* __restrict__ counters /* 1: node count, 2: tri count, 3: error */,
                            uint32_t node_cap, uint32_t tri_cap,
                            const BinNode* __restrict__ bin, const WidePlan* __restrict__ plan,
                            const uint32_t* __restrict__ order, const float3* __restrict__ blo, const float3* __restrict__ bhi,
                            const FFTri* __restrict__ rec, FFNode8* __restrict__ wnodes, FFTri* __restrict__ wtris)
 {
     uint32_t it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= n_in) return;
+    if (it >= level[0] || counters[3]) return;   // (an earlier level's error: its items may be missing)
     CollapseItem item = in[it];
 
     ChildInfo ch[8];
@@ -483,7 +498,7 @@ __global__ void k_collapse(const CollapseItem* __restrict__ in, uint32_t n_in, C
     }
     uint32_t child_base = n_internal ? atomicAdd(&counters[1], n_internal) : 0;
     uint32_t tri_base = n_tris ? atomicAdd(&counters[2], n_tris) : 0;
-    uint32_t out_base = n_internal ? atomicAdd(&counters[0], n_internal) : 0;
+    uint32_t out_base = n_internal ? atomicAdd(&level[1], n_internal) : 0;
     // Capacity guards: a correct build never trips them; if one does, the
     // error flag is set and nothing is written out of bounds.
     if (child_base + n_internal > node_cap || tri_base + n_tris > tri_cap || out_base + n_internal > node_cap ||
@@ -583,14 +598,15 @@ __global__ void k_validate_refs(const uint32_t* __restrict__ tri_refs, uint32_t 
     if (i < n && tri_refs[i] != 1u) atomicAdd(err, 1u);
 }
 
-// Collapse counters (k_collapse): no items out, the root's node taken, no
-// triangles, no error.
-__global__ void k_reset_collapse(uint32_t* c)
+// Collapse counters (k_collapse): the root's node taken, no triangles, no
+// error, and one item, the root, in the first level.
+__global__ void k_reset_collapse(uint32_t* c, uint32_t* level, CollapseItem* queue, CollapseItem root)
 {
-    c[0] = 0;
     c[1] = 1;
     c[2] = 0;
     c[3] = 0;
+    for (int i = 0; i < kMaxLevels + 1; ++i) level[i] = i == 0;
+    *queue = root;
 }
 
 __global__ void k_init_counters(int* cb)
@@ -627,7 +643,8 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
     uint64_t* keys2 = temp.get<uint64_t>(n);
     uint32_t* vals = temp.get<uint32_t>(n);
     uint32_t* vals2 = temp.get<uint32_t>(n);
-    uint32_t* counters = temp.get<uint32_t>(64);
+    uint32_t* counters = temp.get<uint32_t>(64 + kMaxLevels + 1);
+    uint32_t* level = counters + 64;
     int* cb = reinterpret_cast<int*>(counters + 16);
 
     const int B = 256;
@@ -665,27 +682,30 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
     // not do, the collapse runs again with that one.
     s->tris.alloc(sizeof(FFTri) * n);
     uint32_t depth = 0;
-    uint32_t host_counters[4];
+    uint32_t host_counters[64 + kMaxLevels + 1];
     for (uint32_t max_wide : {n / 2 + 2, n + 1}) {
         s->nodes.alloc(sizeof(FFNode8) * max_wide);
         CollapseItem* qin = temp.get<CollapseItem>(max_wide);
         CollapseItem* qout = temp.get<CollapseItem>(max_wide);
-        k_reset_collapse<<<1, 1, 0, st>>>(counters);
-        CollapseItem root{n > 1 ? 0 : ~0, 0u};
-        FF_CUDA_CHECK(cudaMemcpyAsync(qin, &root, sizeof(root), cudaMemcpyHostToDevice, st));
-        host_counters[3] = 0;
+        k_reset_collapse<<<1, 1, 0, st>>>(counters, level, qin, CollapseItem{n > 1 ? 0 : ~0, 0u});
         depth = 0;
-        for (uint32_t n_in = 1; n_in > 0 && !host_counters[3]; std::swap(qin, qout)) {
-            FF_CUDA_CHECK(cudaMemsetAsync(counters, 0, sizeof(uint32_t), st));
-            k_collapse<<<(n_in + 127) / 128, 128, 0, st>>>(
-                qin, n_in, qout, counters, max_wide, n, bin, plan, order, blo,
-                bhi, rec, s->nodes.as<FFNode8>(), s->tris.as<FFTri>());
+        // An item below the root holds more than kLeafMax triangles, and none
+        // of another's: bounds on a level's items besides 8 per item above.
+        const uint64_t most = std::min<uint64_t>(n / (kLeafMax + 1) + 1, max_wide);
+        for (uint64_t n_in = 1; n_in > 0; n_in = host_counters[64 + depth]) {
+            if (depth == kMaxLevels) throw FFError{FF_ERR_INTERNAL, "BVH collapse did not terminate"};
+            for (int k = 0; k < kLevelsAhead; ++k, std::swap(qin, qout)) {
+                k_collapse<<<(uint32_t)((n_in + kCollapseBlock - 1) / kCollapseBlock), kCollapseBlock, 0, st>>>(
+                    qin, qout, level + depth, counters, max_wide, n, bin, plan, order, blo, bhi, rec,
+                    s->nodes.as<FFNode8>(), s->tris.as<FFTri>());
+                ++depth;
+                n_in = std::min(8 * n_in, most);
+            }
             FF_CUDA_CHECK(cudaMemcpyAsync(host_counters, counters, sizeof(host_counters), cudaMemcpyDeviceToHost, st));
             FF_CUDA_CHECK(cudaStreamSynchronize(st));
-            ++depth;
-            n_in = host_counters[0];
-            if (depth > 200) throw FFError{FF_ERR_INTERNAL, "BVH collapse did not terminate"};
+            if (host_counters[3]) break;
         }
+        while (depth > 0 && host_counters[64 + depth - 1] == 0) --depth;   // (levels launched ahead of need)
         if (!host_counters[3]) break;
     }
     if (host_counters[3]) throw FFError{FF_ERR_INTERNAL, "BVH collapse exceeded its capacity"};
