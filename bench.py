@@ -62,13 +62,13 @@ NODE_BYTES, TRI_BYTES = 80, 48
 WF_CLOSEST_BYTES, WF_ANY_BYTES = 32 + 4 + 16, 32 + 4 + 1
 # k_logic in the adjoint, per consumed extension hit: reads the slot words
 # (12 B), the hit (16), the ray record (32), throughput (16), sum and
-# compensation (32), the shading and light-term records (64), the triangle's
-# shading attributes (64), the vertex's derivative terms (albedo + flags, uv,
-# env coefficient, light direction: 56) and, once the sample ends, its vertex
-# record (32); writes sum, compensation, throughput and state (52), the next
-# vertex (64) and the vertex record (32): 472 B.  Every path is traced once;
-# the reported rays count it twice, as an adjoint that replays does.
-ADJ_LOGIC_BYTES_PER_HIT = 472
+# compensation (32) and the shading record (32), writes sum, compensation and
+# state (36): 176 B.  At the 0.72 of the hits that a path goes on from: the
+# triangle's shading attributes (64), the vertex's derivative terms (56),
+# throughput (16), the next vertex (64), its record written (32) and read once
+# the sample ends (32): 264 B.  Every path is traced once; the reported rays
+# count it twice, as for an adjoint that replays.
+ADJ_LOGIC_BYTES_PER_HIT = 366
 ADJ_PASSES_REPORTED = 2
 # k_logic in ff_render, per consumed extension hit of a continuing path:
 # reads the slot words (8 B), the hit (16), the ray record (32), throughput,
@@ -102,8 +102,8 @@ RENDER = dict(width=1920, height=1080, spp=64, max_depth=8, rr_depth=3)
 # Measured DRAM bytes per unit of the adjoint's stages (ncu over the profiled
 # 512x512, 16-spp adjoint call of --workload inverse, 12 frames): per
 # consumed extension hit for k_logic and k_shade, per traced ray for the traces.
-ADJ_DRAM_BYTES_PER_UNIT = {"k_logic (adjoint)": 334.1, "k_shade (adjoint)": 259.2,
-                           "k_trace closest (extension)": 52.0, "k_trace any (shadow)": 39.9}
+ADJ_DRAM_BYTES_PER_UNIT = {"k_logic (adjoint)": 378.8, "k_shade (adjoint)": 173.3,
+                           "k_trace closest (extension)": 48.8, "k_trace any (shadow)": 93.7}
 # k_cache_infer: measured DRAM bytes per query (ncu over 6 cached 1080p
 # frames, 9,513,224 queries): the 64 B record in and the film update; the
 # hash grid's FP16 copy stays in L2.
@@ -1136,7 +1136,7 @@ def inverse_e2e(ctx, dev, stream, iters=5, res=512):
 def inverse_cpu_baseline(target_s=15.0):
     """The oracle's path tracer (C restatement, all host threads) on the same
     scene: primal samples per second over a pixel subset, the lower bound of a
-    CPU adjoint sample's cost (the replay traces every path twice)."""
+    CPU adjoint sample's cost."""
     try:
         from oracle import ffo
     except Exception:
