@@ -40,3 +40,17 @@ def test_few_rays_equal_many(sets, scene, kind):
     for n in (1, 2, 15, 16, 17, 1000, 40960, 40961):
         few = ds.trace(r[:n], **kw)
         assert np.array_equal(few.view(np.uint32), many[:n].view(np.uint32)), n
+
+
+@pytest.mark.parametrize("kind", ["closest", "two_sided", "any"])
+def test_rays_taken_by_the_pool(sets, kind):
+    """Sets large enough for the warps to take 64 rays at a time, ending at and
+    around the sizes where they begin to (two rays a resident thread): the
+    60,000 rays over and over give each time the bits that they give alone."""
+    ds, rays, anyr = sets["room"]
+    r = anyr if kind == "any" else rays
+    kw = dict(any_hit=kind == "any", two_sided=kind == "two_sided")
+    one = ds.trace(r, **kw).view(np.uint32)
+    for n in (606_207, 606_208, 606_273, 1_000_003):
+        got = ds.trace(r[np.arange(n) % len(r)], **kw).view(np.uint32)
+        assert np.array_equal(got, one[np.arange(n) % len(r)]), n
