@@ -50,7 +50,7 @@ def test_rays_taken_by_the_pool(sets, kind):
     ds, rays, anyr = sets["room"]
     r = anyr if kind == "any" else rays
     kw = dict(any_hit=kind == "any", two_sided=kind == "two_sided")
-    one = ds.trace(r, **kw).view(np.uint32)
+    one = ds.trace(r, **kw).view(np.uint32).reshape(-1, 4)
     for n in (606_207, 606_208, 606_273, 1_000_003):
-        got = ds.trace(r[np.arange(n) % len(r)], **kw).view(np.uint32)
+        got = ds.trace(r[np.arange(n) % len(r)], **kw).view(np.uint32).reshape(-1, 4)
         assert np.array_equal(got, one[np.arange(n) % len(r)]), n
