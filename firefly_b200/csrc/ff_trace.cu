@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8)
                 }
             }
         }
+        __syncwarp();   // (votes order no memory: lane 0's push before the group's pop below)
         const uint32_t kids = (__ballot_sync(0xffffffffu, inner) >> first) & 0xffu;
 #pragma unroll
         for (uint32_t k = 1; k < kGroup; k <<= 1) tmask |= __shfl_xor_sync(0xffffffffu, tmask, k);
