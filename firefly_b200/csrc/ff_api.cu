@@ -131,8 +131,8 @@ ff_status ff_context_create(const ff_device_opts* opts, ff_context** out)
             FF_CUDA_CHECK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
             ctx->own_stream = true;
         }
-        ctx->counters.alloc(256);
-        FF_CUDA_CHECK(cudaMemsetAsync(ctx->counters.ptr, 0, 256, ctx->stream));
+        ctx->small.alloc(ff_context::kCounterBytes + ff_context::kSmallRays * (sizeof(ff_ray) + sizeof(ff_hit)));
+        FF_CUDA_CHECK(cudaMemsetAsync(ctx->counters(), 0, ff_context::kCounterBytes, ctx->stream));
         FF_CUDA_CHECK(cudaEventCreate(&ctx->ev0));
         FF_CUDA_CHECK(cudaEventCreate(&ctx->ev1));
     });
@@ -152,10 +152,9 @@ ff_status ff_context_destroy(ff_context* ctx)
         cudaGetDevice(&prev);
         cudaSetDevice(ctx->device);
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-        ctx->counters.release();
+        ctx->small.release();
         ctx->io_rays.release();
         ctx->io_hits.release();
-        ctx->io_small.release();
         ctx->scratch.release();
         if (ctx->io_pin) cudaFreeHost(ctx->io_pin);
         for (auto& b : ctx->adj_io) b.release();
@@ -307,33 +306,38 @@ namespace {
 // Rays per chunk of a host-pointer trace: 64 MB in, 32 MB out.
 constexpr uint64_t kIoChunk = 1ull << 21;
 
-// Host-pointer traces of up to this many rays go through pinned staging.
-constexpr uint64_t kIoSmall = 8192;
+// The pinned staging of small host-pointer traces; false where the system
+// grants none (they then go the way of large ones).
+bool small_staging(ff_context* ctx)
+{
+    if (ctx->io_pin) return true;
+    if (cudaMallocHost(&ctx->io_pin, ctx->small.bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    ctx->io_pin = nullptr;
+    return false;
+}
 
-// A small host-pointer trace: one copy in (the zeroed ray counter, the rays,
-// the zeroed error count), the trace, one copy out (the error count, the
-// hits), through pinned staging that the context keeps.  Three copies from
-// and to pageable memory, a memset and two more streams' events took 67 us
-// for 100 rays, this 45.  Synchronous; returns the error count.
+// A small host-pointer trace: one copy in (the rays, a zero ray counter), the
+// trace, one copy out (the error count, the hits), through pinned staging that
+// the context keeps.  Three copies from and to pageable memory, a memset and
+// two more streams' events took 67 us for 100 rays, this 45.  Synchronous;
+// returns the context's error count.
 unsigned int trace_host_small(ff_context* ctx, const ff_scene* s, const ff_ray* rays, uint64_t n, ff_hit* hits, bool any,
                               bool two)
 {
-    constexpr size_t kBytes = 32 + kIoSmall * (sizeof(ff_ray) + sizeof(ff_hit));
-    ctx->io_small.alloc(kBytes);
-    if (!ctx->io_pin) FF_CUDA_CHECK(cudaMallocHost(&ctx->io_pin, kBytes));
-    char *pin = ctx->io_pin, *dev = ctx->io_small.as<char>();
-    const size_t at_err = 16 + n * sizeof(ff_ray), at_hits = at_err + 16;
-    std::memset(pin, 0, 16);
-    std::memcpy(pin + 16, rays, n * sizeof(ff_ray));
-    std::memset(pin + at_err, 0, 16);
-    FF_CUDA_CHECK(cudaMemcpyAsync(dev, pin, at_hits, cudaMemcpyHostToDevice, ctx->stream));
-    ff_launch_trace_scratch(ctx, s, reinterpret_cast<ff_ray*>(dev + 16), n, reinterpret_cast<ff_hit*>(dev + at_hits), any,
-                            reinterpret_cast<unsigned long long*>(dev), reinterpret_cast<unsigned int*>(dev + at_err), two);
-    FF_CUDA_CHECK(cudaMemcpyAsync(pin + at_err, dev + at_err, 16 + n * sizeof(ff_hit), cudaMemcpyDeviceToHost, ctx->stream));
+    char *dev = ctx->counters(), *pin = ctx->io_pin + (dev - ctx->small.as<char>());
+    constexpr size_t at_err = ff_context::kTraceErr, at_hits = ff_context::kCounterBytes;
+    const size_t in = n * sizeof(ff_ray), out = n * sizeof(ff_hit);
+    std::memcpy(pin - in, rays, in);
+    std::memset(pin, 0, at_err);
+    FF_CUDA_CHECK(cudaMemcpyAsync(dev - in, pin - in, in + at_err, cudaMemcpyHostToDevice, ctx->stream));
+    ff_launch_trace_scratch(ctx, s, reinterpret_cast<ff_ray*>(dev - in), n, reinterpret_cast<ff_hit*>(dev + at_hits), any,
+                            reinterpret_cast<unsigned long long*>(dev), ctx->trace_err(), two);
+    FF_CUDA_CHECK(cudaMemcpyAsync(pin + at_err, dev + at_err, at_hits - at_err + out, cudaMemcpyDeviceToHost, ctx->stream));
     FF_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
     unsigned int err;
     std::memcpy(&err, pin + at_err, sizeof(err));
-    std::memcpy(hits, pin + at_hits, n * sizeof(ff_hit));
+    std::memcpy(hits, pin + at_hits, out);
     return err;
 }
 
@@ -406,19 +410,19 @@ ff_status ff_trace(ff_context* ctx, const ff_scene* s, const ff_ray* rays, uint6
             FF_REQUIRE((reinterpret_cast<uintptr_t>(rays) & 15) == 0 && (reinterpret_cast<uintptr_t>(hits) & 15) == 0,
                        "device rays and hits must be 16-byte aligned");
             ff_launch_trace(ctx, s, rays, n, hits, any, two);
-        } else if (n <= kIoSmall) {
-            if (trace_host_small(ctx, s, rays, n, hits, any, two))
-                throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
         } else {
-            ctx->io_rays.alloc(sizeof(ff_ray) * n);
-            ctx->io_hits.alloc(sizeof(ff_hit) * n);
-            trace_host_chunks(ctx, s, rays, n, hits, any, two);
             unsigned int err = 0;
-            FF_CUDA_CHECK(cudaMemcpyAsync(&err, ctx->counters.as<char>() + 8, sizeof(err), cudaMemcpyDeviceToHost,
-                                          ctx->stream));
-            FF_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-            if (err) {
-                FF_CUDA_CHECK(cudaMemsetAsync(ctx->counters.as<char>() + 8, 0, sizeof(err), ctx->stream));
+            if (n <= ff_context::kSmallRays && small_staging(ctx)) {
+                err = trace_host_small(ctx, s, rays, n, hits, any, two);
+            } else {
+                ctx->io_rays.alloc(sizeof(ff_ray) * n);
+                ctx->io_hits.alloc(sizeof(ff_hit) * n);
+                trace_host_chunks(ctx, s, rays, n, hits, any, two);
+                FF_CUDA_CHECK(cudaMemcpyAsync(&err, ctx->trace_err(), sizeof(err), cudaMemcpyDeviceToHost, ctx->stream));
+                FF_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+            }
+            if (err) {   // of this call or of device-pointer calls before it
+                FF_CUDA_CHECK(cudaMemsetAsync(ctx->trace_err(), 0, sizeof(err), ctx->stream));
                 throw FFError{FF_ERR_INTERNAL, "traversal exceeded its step bound (malformed BVH)"};
             }
         }
@@ -448,9 +452,8 @@ ff_status ff_trace_count(ff_context* ctx, const ff_scene* s, const ff_ray* rays,
                                           ctx->stream));
             d_rays = ctx->io_rays.as<ff_ray>();
         }
-        // counters: [16..31] the two work totals, [8..11] the traversal error count
-        unsigned long long* d_out = reinterpret_cast<unsigned long long*>(ctx->counters.as<char>() + 16);
-        unsigned int* err = reinterpret_cast<unsigned int*>(ctx->counters.as<char>() + 8);
+        unsigned long long* d_out = reinterpret_cast<unsigned long long*>(ctx->counters() + ff_context::kCounterBytes);
+        unsigned int* err = ctx->trace_err();
         FF_CUDA_CHECK(cudaMemsetAsync(d_out, 0, 2 * sizeof(unsigned long long), ctx->stream));
         ff_launch_trace_count(ctx, s, d_rays, n, any, d_out, err, two);
         unsigned long long h[2] = {0, 0};
@@ -542,6 +545,16 @@ extern "C" ff_status ff_debug_alloc_stats(uint64_t* total, int64_t* live)
     if (total) *total = g_ff_alloc.total.load();
     if (live) *live = g_ff_alloc.live.load();
     return FF_OK;
+}
+
+extern "C" ff_status ff_debug_trace_errors(ff_context* ctx, uint32_t count)
+{
+    if (!ctx) return FF_ERR_INVALID_ARG;
+    return guarded(ctx, [&] {
+        DeviceGuard g(ctx->device);
+        FF_CUDA_CHECK(cudaMemcpyAsync(ctx->trace_err(), &count, sizeof(count), cudaMemcpyHostToDevice, ctx->stream));
+        FF_CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    });
 }
 
 extern "C" ff_status ff_debug_fail_alloc_after(int64_t n)

@@ -158,13 +158,20 @@ struct ff_context {
     bool own_stream = false;
     int num_sms = 148;
     std::string last_error;
-    DevBuf counters;      // small scratch of uint32 counters for persistent kernels
+    // Counters of the traces that take the context's: the ray counter and, at
+    // kTraceErr, the traversal error count (sticky until a host-pointer call
+    // reports it).  Before them is room for the rays of a small host-pointer
+    // trace, ending where the counters begin, after them for its hits: one copy
+    // brings in the rays and a zero ray counter, one takes out the error count
+    // and the hits.  (ff_trace_count keeps its totals where the hits go.)
+    DevBuf small;
+    static constexpr uint64_t kSmallRays = 8192;
+    static constexpr size_t kTraceErr = 16, kCounterBytes = 32;
+    char* counters() const { return small.as<char>() + kSmallRays * sizeof(ff_ray); }
+    unsigned int* trace_err() const { return reinterpret_cast<unsigned int*>(counters() + kTraceErr); }
     FFScratch scratch;        // temporaries of scene and table builds
     DevBuf io_rays, io_hits;  // staging for host-pointer ff_trace calls
-    // staging of small host-pointer traces: pinned host memory and its device
-    // counterpart (created on first use)
-    char* io_pin = nullptr;
-    DevBuf io_small;
+    char* io_pin = nullptr;   // pinned counterpart of `small` (created on first use)
     // host-pointer ff_trace: rays copied in on io_in, hits copied out on
     // io_out, each chunk's trace on `stream` between them (created on first use)
     cudaStream_t io_in = nullptr, io_out = nullptr;

@@ -462,10 +462,8 @@ void ff_launch_trace(ff_context* ctx, const ff_scene* s, const ff_ray* d_rays, u
                      bool any_hit, bool two_sided)
 {
     if (n == 0) return;
-    unsigned long long* counter = ctx->counters.as<unsigned long long>();
-    // counters: [0..7] ray counter, [8..11] traversal error count (sticky
-    // until read by ff_trace_errors / the host-pointer path)
-    unsigned int* err = reinterpret_cast<unsigned int*>(ctx->counters.as<char>() + 8);
+    unsigned long long* counter = reinterpret_cast<unsigned long long*>(ctx->counters());
+    unsigned int* err = ctx->trace_err();
     FF_CUDA_CHECK(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), ctx->stream));
     launch_trace(ctx, s->view(), d_rays, n, d_hits, any_hit, two_sided, counter, err, nullptr, nullptr, nullptr,
                  ctx->stream, 0);

@@ -516,6 +516,10 @@ FF_API ff_status ff_debug_alloc_stats(uint64_t* total, int64_t* live);
  * every later one fails with FF_ERR_OOM, without calling cudaMalloc; n < 0
  * turns the refusal off.  Process-wide. */
 FF_API ff_status ff_debug_fail_alloc_after(int64_t n);
+/* Sets the context's traversal error count, as device-pointer ff_trace calls
+ * over a malformed BVH would leave it; the next ff_trace or ff_trace_count that
+ * waits for the device reports it (FF_ERR_INTERNAL) and clears it. */
+FF_API ff_status ff_debug_trace_errors(ff_context* ctx, uint32_t count);
 /* Bound of the radiance cache's tensor-core waits, in polls of the
  * mbarrier (0: every wait gives up at once; FF_DEBUG_WAIT_DEFAULT: the
  * built-in bound).  A wait that gives up makes the call return
