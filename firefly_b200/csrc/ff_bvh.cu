@@ -16,6 +16,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 
 #include "ff_internal.h"
@@ -439,6 +440,26 @@ __global__ void __launch_bounds__(kCollapseBlock)
             }
             if (j) open(ref, j, i - j);
             else ch[nc++] = info(ref);
+        }
+        // Where a box has no area (triangles on a line or in a point) or its
+        // area overflows (extents above 1e19), every split costs the same and
+        // the plan has none: there the subtree with the most triangles is
+        // opened until the slots are used, or the tree stays binary.
+        while (nc < 8) {
+            int most = -1;
+            uint32_t count = kLeafMax;
+            for (int c = 0; c < nc; ++c) {
+                const uint32_t cnt = ch[c].last - ch[c].first + 1;
+                const float a = half_area(ch[c].lo, ch[c].hi);
+                if (cnt > count && !(a > 0.f && a <= FLT_MAX)) {
+                    most = c;
+                    count = cnt;
+                }
+            }
+            if (most < 0) break;
+            const BinNode& b = bin[ch[most].ref];
+            ch[nc++] = info(b.right);
+            ch[most] = info(b.left);
         }
     }
 
