@@ -375,6 +375,10 @@ void ff_adjoint_render(ff_context* ctx, ff_scene* scene, const ff_render_setting
     FF_REQUIRE(st->light != FF_LIGHT_ALL, "the adjoint needs one light (FF_LIGHT_ALL is not supported)");
     ff_check_light(scene, st->light, FF_MODE_CORRECTED);
     cudaStream_t stream = ctx->stream;
+    struct Records {   // whose use ends with the call, however it ends
+        ff_context* ctx;
+        ~Records() { ff_wavefront_records_idle(ctx->adj_ws); }
+    } records{ctx};
     const bool dev = (ad->flags & FF_MEM_DEVICE) != 0;
     const size_t npix = (size_t)ad->width * ad->height;
     const bool rough = ad->grad_roughness != nullptr;

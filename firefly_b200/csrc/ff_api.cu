@@ -19,6 +19,7 @@ thread_local std::string g_create_error;
 template <class F>
 ff_status guarded(ff_context* ctx, F&& f)
 {
+    FFCall call(ctx);
     try {
         f();
         return FF_OK;
@@ -107,6 +108,18 @@ void ff_build_env_tables(ff_context* ctx, ff_scene* s);
 void ff_env_pack(ff_context* ctx, ff_scene* s);
 void ff_build_shading(ff_context* ctx, ff_scene* s, const ff_scene_desc* d, const float3* d_pos,
                       const uint3* d_idx);
+
+thread_local ff_context* t_ff_call = nullptr;
+
+bool ff_give_back(ff_context* ctx)
+{
+    bool any = ff_wavefront_records_release(ctx->adj_ws);
+    if (ctx->scratch.scopes == 0 && !ctx->scratch.blocks.empty()) {
+        ctx->scratch.release();
+        any = true;
+    }
+    return any;
+}
 
 extern "C" {
 

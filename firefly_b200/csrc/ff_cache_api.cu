@@ -9,6 +9,7 @@ namespace {
 template <class F>
 ff_status cache_guard(ff_context* ctx, F&& f)
 {
+    FFCall call(ctx);
     try {
         int prev = -1;
         cudaGetDevice(&prev);

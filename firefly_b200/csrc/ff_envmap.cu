@@ -230,6 +230,7 @@ extern "C" ff_status ff_debug_env_pick(const ff_scene* scene, const float* exy, 
         ctx->last_error = "ff_debug_env_pick: more than 2^32 draws";
         return FF_ERR_INVALID_ARG;
     }
+    FFCall call(ctx);
     try {
         FF_CUDA_CHECK(cudaSetDevice(ctx->device));
         cudaStream_t st = ctx->stream;

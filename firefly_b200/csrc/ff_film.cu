@@ -46,6 +46,7 @@ __global__ void k_resolve(const float4* __restrict__ acc, const float4* __restri
 template <class F>
 ff_status film_guard(ff_film* f, F&& fn)
 {
+    FFCall call(f->ctx);
     try {
         fn();
         return FF_OK;

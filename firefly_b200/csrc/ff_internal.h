@@ -56,6 +56,20 @@ inline bool ff_alloc_refused()
     return false;
 }
 
+// The context that the calling thread's API call works on.  What a context
+// keeps from call to call and can do without (ff_give_back: the temporaries'
+// block, the adjoint's vertex records) goes back to the device when an
+// allocation of one of its calls is refused, before that call fails.
+extern thread_local ff_context* t_ff_call;
+struct FFCall {
+    ff_context* outer;
+    explicit FFCall(ff_context* ctx) : outer(t_ff_call) { t_ff_call = ctx; }
+    ~FFCall() { t_ff_call = outer; }
+    FFCall(const FFCall&) = delete;
+    FFCall& operator=(const FFCall&) = delete;
+};
+bool ff_give_back(ff_context* ctx);   // whether there was anything
+
 // Device allocation: owned, or a place in another buffer.
 struct DevBuf {
     void* ptr = nullptr;
@@ -88,8 +102,17 @@ struct DevBuf {
         if (n <= bytes && ptr) return;
         release();
         if (n == 0) return;
-        if (ff_alloc_refused()) throw FFError{FF_ERR_OOM, "device allocation refused (ff_debug_fail_alloc_after)"};
-        FF_CUDA_CHECK(cudaMalloc(&ptr, n));
+        for (bool again = true;; again = false) {
+            if (!ff_alloc_refused()) {
+                const cudaError_t e = cudaMalloc(&ptr, n);
+                if (e == cudaSuccess) break;
+                cudaGetLastError();   // (or the next launch would report it)
+                ptr = nullptr;
+                if (e != cudaErrorMemoryAllocation) FF_CUDA_CHECK(e);
+            }
+            if (!again || !t_ff_call || !ff_give_back(t_ff_call))
+                throw FFError{FF_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes refused"};
+        }
         g_ff_alloc.total.fetch_add(1);
         g_ff_alloc.live.fetch_add(1);
         bytes = n;
@@ -103,7 +126,7 @@ struct DevBuf {
 // cudaFree cost 0.1 to 0.3 ms each and the free waits for the device: 35 of
 // both were over 80% of a scene's load (81,932 triangles under a 1024 x 512
 // sky: 9.8 ms, now 2.4).  Between calls one block of at most kKeep bytes stays; the
-// context frees it.  Every use is on the context's stream and calls on a
+// context frees it, or ff_give_back.  Every use is on the context's stream and calls on a
 // context are externally serialised, so a block is reused in order.
 struct FFScratch {
     static constexpr size_t kKeep = 256ull << 20, kMinBlock = 8ull << 20;
@@ -151,6 +174,10 @@ struct FFScratch {
 
 struct FFWavefrontWS;
 void ff_wavefront_ws_free(FFWavefrontWS* ws);
+// The adjoint's vertex records between calls: ff_wavefront_records_idle ends a
+// call's use of them, ff_wavefront_records_release frees what no call is using.
+void ff_wavefront_records_idle(FFWavefrontWS* ws);
+bool ff_wavefront_records_release(FFWavefrontWS* ws);
 
 struct ff_context {
     int device = 0;

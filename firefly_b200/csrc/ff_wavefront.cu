@@ -874,6 +874,7 @@ struct FFWavefrontWS {
     DevBuf buf;
     DevBuf adj_buf;   // the adjoint's per-slot arrays (allocated by ff_wavefront_adjoint only)
     DevBuf rec_buf;   // the adjoint's vertex records
+    bool rec_idle = true;   // no call is using them
     DevBuf defer_buf; // the deferred light terms' arrays (allocated by ff_render only)
     uint32_t defer_P = 0;
     uint64_t next_stamp = kFirstStamp;   // the first stamp the next render may use
@@ -951,6 +952,24 @@ struct FFWavefrontWS {
 };
 
 void ff_wavefront_ws_free(FFWavefrontWS* ws) { delete ws; }
+
+bool ff_wavefront_records_release(FFWavefrontWS* ws)
+{
+    if (!ws || !ws->rec_idle || !ws->rec_buf.ptr) return false;
+    ws->rec_buf.release();
+    return true;
+}
+
+// Records of up to this many bytes stay for the next call (an optimiser's
+// steps); allocating and freeing more costs little beside the call that uses it.
+constexpr size_t kRecordKeep = 1ull << 30;
+
+void ff_wavefront_records_idle(FFWavefrontWS* ws)
+{
+    if (!ws) return;
+    ws->rec_idle = true;
+    if (ws->rec_buf.bytes > kRecordKeep) ws->rec_buf.release();
+}
 
 namespace {
 
@@ -1385,7 +1404,8 @@ namespace {
 
 // Records of the adjoint's vertices are kept up to this many bytes, else
 // every sample is replayed.  At 512 x 512 x 16
-// samples, depth 3 with an albedo texture, they take 0.4 GB.
+// samples, depth 3 with an albedo texture, they take 0.4 GB.  What stays
+// allocated after the call: kRecordKeep, and until an allocation is refused.
 constexpr uint64_t kRecordBudget = 4ull << 30;
 
 // The adjoint's per-slot arrays, and the records where they fit the budget
@@ -1420,9 +1440,9 @@ void adj_setup(FFWavefrontWS* ws, uint32_t P, uint32_t max_depth, bool albedo, b
         ws->rec_buf.alloc(albedo || rough ? bytes : 256u);
     } catch (const FFError& e) {
         if (e.status != FF_ERR_OOM) throw;
-        cudaGetLastError();
         return;
     }
+    ws->rec_idle = false;   // (until ff_wavefront_records_idle)
     p = ws->rec_buf.as<char>();
     w.rec0 = w.rec1 = reinterpret_cast<float4*>(p);   // (only the environment takes gradients: nothing is kept)
     if (!albedo && !rough) return;
