@@ -170,7 +170,7 @@ class dScene:
                        grad_env=None, spp: int = 1, max_depth: int = 3, rr_depth: int = 3, seed: int = 0,
                        light: int = -1, sample_offset: int = 0, shadow_offset: float = 0.001,
                        store_all: bool = False, roughness_texture: int = -1, grad_roughness=None,
-                       megakernel: bool = False, profile: bool = False) -> dict:
+                       megakernel: bool = False, profile: bool = False, replay: bool = False) -> dict:
         """Path-replay adjoint of PathTracer.draw(mode=FF_MODE_CORRECTED) with
         the same settings: adds dL/d(texture texels) to grad_texture,
         dL/d(env texels) to grad_env and dL/d(roughness texels) to
@@ -178,9 +178,11 @@ class dScene:
         channel 0 where a material reads the texture as its roughness_tex,
         channel 1 where it is the packed metallic_roughness_tex), given
         d_image = dL/dI of the mean-radiance image (height, width, 3).
-        The replay runs on the wavefront stages; megakernel=True runs the
-        one-thread-per-sample replay instead, store_all=True the store-all
-        reference variant.  profile=True times the wavefront stages
+        The adjoint runs on the wavefront stages, with each sample's vertices
+        kept until its radiance is known, or, with replay=True or where they
+        take too much memory, with every sample replayed from its seed;
+        megakernel=True runs the one-thread-per-sample replay instead,
+        store_all=True the store-all reference variant.  profile=True times the wavefront stages
         (ms_logic, ms_shade, ms_trace_extension, ms_trace_shadow)."""
         dimg = np.ascontiguousarray(d_image, np.float32)
         s = A.ff_render_settings(spp=spp, max_depth=max_depth, rr_depth=rr_depth, seed=seed,
@@ -190,7 +192,8 @@ class dScene:
                               grad_texture=None if grad_texture is None else grad_texture.ctypes.data,
                               grad_env=None if grad_env is None else grad_env.ctypes.data,
                               flags=(A.FF_ADJOINT_STORE_ALL if store_all else 0)
-                              | (A.FF_ADJOINT_MEGAKERNEL if megakernel else 0),
+                              | (A.FF_ADJOINT_MEGAKERNEL if megakernel else 0)
+                              | (A.FF_ADJOINT_REPLAY if replay else 0),
                               roughness_texture=roughness_texture,
                               grad_roughness=None if grad_roughness is None else grad_roughness.ctypes.data)
         for g in (grad_texture, grad_env, grad_roughness):

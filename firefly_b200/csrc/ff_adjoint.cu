@@ -455,9 +455,10 @@ void ff_adjoint_render(ff_context* ctx, ff_scene* scene, const ff_render_setting
     FF_REQUIRE(!mega || blocks < (1ull << 31), "adjoint launch too large");
     FF_CUDA_CHECK(cudaEventRecord(ctx->ev0, stream));
     if (!mega) {
-        // the default: path replay on the wavefront stages
+        // the default: the wavefront stages
         FFAdjointTarget t{ad->width, ad->height, d_image, ad->texture, ntex ? g_tex : nullptr, a.grad_env,
-                          a.rough_texture, a.grad_rough, ctr.as<unsigned long long>() + 2};
+                          a.rough_texture, a.grad_rough, ctr.as<unsigned long long>() + 2,
+                          (ad->flags & FF_ADJOINT_REPLAY) != 0};
         ff_wavefront_adjoint(ctx, scene, st, t, stats);
     } else if (store_all && rough) {
         k_adjoint<true, true><<<(unsigned)blocks, kAdjBlock, 0, stream>>>(a);

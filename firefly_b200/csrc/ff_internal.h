@@ -383,6 +383,7 @@ struct FFAdjointTarget {
     int32_t rough_texture;
     float* grad_rough;
     unsigned long long* touched;
+    bool replay;
 };
 void ff_wavefront_adjoint(ff_context* ctx, ff_scene* scene, const ff_render_settings* st, const FFAdjointTarget& t,
                           ff_render_stats* stats);

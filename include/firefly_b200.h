@@ -349,6 +349,8 @@ FF_API ff_status ff_render(ff_context* ctx, ff_scene* scene, const ff_render_set
 #define FF_ADJOINT_STORE_ALL 4u   /* ff_adjoint_desc.flags: store-all-vertices reference variant */
 #define FF_ADJOINT_MEGAKERNEL 16u /* ff_adjoint_desc.flags: one-thread-per-sample replay (cross-check) instead of
                                      the wavefront stages */
+#define FF_ADJOINT_REPLAY 32u     /* ff_adjoint_desc.flags: keep no vertices, replay every sample from its seed; gives
+                                     back the memory that earlier calls kept them in */
 #define FF_ENV_KEEP_TABLES   8u   /* ff_scene_set_environment: keep the importance tables */
 
 /* Gradient request of ff_render_adjoint.  d_image is dL/dI for the mean
@@ -373,8 +375,8 @@ typedef struct ff_adjoint_desc {
 /* Adjoint of ff_render (no counterpart in the reference, which renders
  * only): the same paths as ff_render in FF_MODE_CORRECTED for the same
  * settings (seed, spp, sample_offset, depths, light), their vertices kept until
- * the sample's radiance is known, or, where that takes too much memory,
- * replayed from their seeds; gradients of the albedo texture of FF_MAT_DIFFUSE surfaces, of the
+ * the sample's radiance is known, or, where that takes more than 4 GiB or more
+ * than the device has left, or with FF_ADJOINT_REPLAY, replayed from their seeds; gradients of the albedo texture of FF_MAT_DIFFUSE surfaces, of the
  * roughness texture of GGX surfaces (FF_MAT_MIX, CONDUCTOR, DIELECTRIC, COAT)
  * and of the environment map (camera misses and NEE), with detached sampling
  * (directions, pdfs, MIS weights and the roulette are not differentiated).
