@@ -66,10 +66,8 @@ WF_CLOSEST_BYTES, WF_ANY_BYTES = 32 + 4 + 16, 32 + 4 + 1
 # state (36): 176 B.  At the 0.72 of the hits that a path goes on from: the
 # triangle's shading attributes (64), the vertex's derivative terms (56),
 # throughput (16), the next vertex (64), its record written (32) and read once
-# the sample ends (32): 264 B.  Every path is traced once; the reported rays
-# count it twice, as for an adjoint that replays.
+# the sample ends (32): 264 B.
 ADJ_LOGIC_BYTES_PER_HIT = 366
-ADJ_PASSES_REPORTED = 2
 # k_logic in ff_render, per consumed extension hit of a continuing path:
 # reads the slot words (8 B), the hit (16), the ray record (32), throughput,
 # sum and compensation (48), the pending light-term record of two frames back
@@ -1050,9 +1048,8 @@ def inverse_line(args, ws, rank, local, dist, ctx, dev, stream, known_lighting_r
                   "k_trace closest (extension)": prof["ms_trace_extension"],
                   "k_trace any (shadow)": prof["ms_trace_shadow"]}
         r["adjoint_stage_ms"] = {k: round(v, 3) for k, v in stages.items()}
-        r["adjoint_rays"] = {"extension": prof["extension_rays"], "shadow": prof["shadow_rays"]}
-        ext_traced = prof["extension_rays"] // ADJ_PASSES_REPORTED
-        shadow_traced = prof["shadow_rays"] // ADJ_PASSES_REPORTED
+        ext_traced, shadow_traced = adjoint_rays_traced(prof)
+        r["adjoint_rays"] = {"extension": ext_traced, "shadow": shadow_traced}
         dom = max(stages, key=stages.get)
         if dom.startswith("k_logic"):
             # one consumed extension hit per slot and frame
@@ -1089,6 +1086,15 @@ def inverse_line(args, ws, rank, local, dist, ctx, dev, stream, known_lighting_r
                 "cpu_baseline": cpu, "e2e": e2e,
                 "gpu_launches": int(round(r["kernel_launches_per_step"] * r["steps"])), "clocks": clk}
     return line if rank == 0 else None
+
+
+def adjoint_rays_traced(st, max_depth=3):
+    """The extension and shadow rays that a profiled adjoint call traced (one
+    sample a slot).  Its statistics count the rays of the forward and of the
+    gradient pass; a call that keeps the vertices traces both as one and needs
+    at most max_depth + 2 frames, a replaying call traces each."""
+    one = st["frames"] <= max_depth + 2
+    return tuple(st[k] // (2 if one else 1) for k in ("extension_rays", "shadow_rays"))
 
 
 def inverse_e2e(ctx, dev, stream, iters=5, res=512):

@@ -314,8 +314,9 @@ typedef struct ff_render_settings {
 } ff_render_settings;
 
 typedef struct ff_render_stats {
-    uint64_t extension_rays;    /* closest-hit queries traced */
-    uint64_t shadow_rays;       /* any-hit queries traced */
+    uint64_t extension_rays;    /* closest-hit queries traced (ff_render_adjoint: of the forward and the gradient
+                                   pass, which are one trace where the vertices are kept) */
+    uint64_t shadow_rays;       /* any-hit queries traced (likewise) */
     uint64_t samples;           /* completed paths */
     uint32_t frames;            /* wavefront iterations */
     float ms_total;
