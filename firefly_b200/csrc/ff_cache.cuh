@@ -36,7 +36,7 @@ struct Grid {
     uint32_t cell_levels;
     uint32_t cell_off[kLevels];
 };
-constexpr uint32_t kCellMax = 1u << 18;   // cells of a level kept by cells (8 MB)
+constexpr uint32_t kCellMax = 1u << 18;   // cells of a level kept by cells (8 MB a level; the default levels have 10 in all)
 
 // One record: a vertex (position, roughness, outgoing direction, normal)
 // and a value (training: target radiance; render queries: path throughput).
