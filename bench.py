@@ -60,26 +60,33 @@ NODE_BYTES, TRI_BYTES = 80, 48
 # The wavefront's traces read a tagged queue (32 B ray + 4 B tag): the
 # closest-hit trace writes a 16 B hit, the any-hit trace a 1 B answer.
 WF_CLOSEST_BYTES, WF_ANY_BYTES = 32 + 4 + 16, 32 + 4 + 1
-# k_logic in the adjoint, per consumed extension hit: reads the slot words
-# (12 B), the hit (16), the ray record (32), throughput (16), sum and
-# compensation (32) and the shading record (32), writes sum, compensation and
-# state (36): 176 B.  At the 0.72 of the hits that a path goes on from: the
-# triangle's shading attributes (64), the vertex's derivative terms (56),
-# throughput (16), the next vertex (64), its record written (32) and read once
-# the sample ends (32): 264 B.
-ADJ_LOGIC_BYTES_PER_HIT = 366
-# k_logic in ff_render, per consumed extension hit of a continuing path:
-# reads the slot words (8 B), the hit (16), the ray record (32), throughput,
-# sum and compensation (48), the pending light-term record of two frames back
-# and its answer word (68) and the triangle's shading attributes (64); writes
-# sum, compensation and state (36) and the vertex record (64): 336 B.
-RENDER_LOGIC_BYTES_PER_HIT = 336
+# Bytes that k_logic cannot do without, per consumed extension hit, per vertex
+# it goes on to (hits less samples) and per started sample.
+# ff_render: a hit reads the slot words (8 B), the hit (16), the ray record
+# (32), throughput (16), sum and compensation (32) and the first half of the
+# pending record of two frames back (32), and writes sum, compensation and
+# state (36): 172.  A vertex reads the answer word of its light terms (4) and
+# the triangle's shading attributes (64) and writes its record (64) and queue
+# entry (4): 136; the pending record's second half is read only where a
+# BSDF-sampled ray was unoccluded and is not counted.  A sample reads and writes
+# its index (8) and writes key, state, throughput and ray (56) and its queue
+# entry (36): 100.
+RENDER_LOGIC_BYTES = {"hit": 172, "vertex": 136, "sample": 100}
+# Adjoint with kept vertices: a hit reads the slot words (12), the hit (16), the
+# ray record (32), throughput (16), sum (16) and dL/dI (12) and writes sum and
+# state (20): 124.  A vertex reads the shading record (32), the albedo (16) and
+# half of the vertex record (32) once its rays are answered, and the triangle's
+# shading attributes (64); its record is written and read back (64), throughput
+# (16), the next vertex (64) and the queue entry (4) are written: 292.  A sample:
+# as above, and sum and count cleared (20): 120.
+ADJ_LOGIC_BYTES = {"hit": 124, "vertex": 292, "sample": 120}
 # k_shade, per shaded vertex: reads the vertex record (64 B), its queue
 # entry (4) and the throughput (16), writes the throughput (16), the ray
-# record (32), the extension-queue entry (36) and the pending light-term
-# record (64): 232 B; plus 36 B per shadow-queue entry (32 B ray, 4 B tag).
+# record (32), the extension-queue entry (36) and the first half of the
+# pending light-term record (32; the second only for BSDF-sampled terms, not
+# counted): 200 B; plus 36 B per shadow-queue entry (32 B ray, 4 B tag).
 # Environment and material lookups are L2 gathers and not counted.
-RENDER_SHADE_BYTES_PER_VERTEX = 232
+RENDER_SHADE_BYTES_PER_VERTEX = 200
 SHADOW_QUEUE_BYTES = 36
 # Measured DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unit
 # of each render stage: ncu over every launch of one timed 16-spp C2 step on
@@ -88,26 +95,31 @@ SHADOW_QUEUE_BYTES = 36
 RENDER_DRAM_BYTES_PER_UNIT = {"k_logic": 343.3, "k_shade (all kinds)": 408.0,
                               "k_trace<closest> (extension queue)": 107.5, "k_trace<any> (shadow queue)": 48.4}
 # Issue slots busy (smsp__issue_active) of the closest-hit traversal on C2:
-# ncu --set full of one steady-state launch of the same 16-spp, 2M-slot step
+# ncu of one steady-state launch of the same 16-spp, 2M-slot step
 # (a figure from that capture, not measured by this run).
-RENDER_ISSUE_SLOTS = {"k_trace<closest> (extension queue)": 0.696}
-# Issue slots busy of the trace micro-benchmark's four launches (ncu --set full
+RENDER_ISSUE_SLOTS = {"k_trace<closest> (extension queue)": 0.730}
+# Issue slots busy of the trace micro-benchmark's four launches (ncu
 # of one launch per batch kind, 4,194,304 rays each; figures from that
 # capture, not measured by this run): the traversal is issue-bound.
-TRACE_ISSUE_SLOTS = {"coherent_closest": 0.835, "incoherent_closest": 0.775, "coherent_any": 0.804,
-                     "incoherent_any": 0.749}
+TRACE_ISSUE_SLOTS = {"coherent_closest": 0.785, "incoherent_closest": 0.776, "coherent_any": 0.809,
+                     "incoherent_any": 0.794}
 RENDER = dict(width=1920, height=1080, spp=64, max_depth=8, rr_depth=3)
 # Measured DRAM bytes per unit of the adjoint's stages (ncu over the profiled
-# 512x512, 16-spp adjoint call of --workload inverse, 12 frames): per
+# 512x512, 16-spp adjoint call of --workload inverse, 5 frames): per
 # consumed extension hit for k_logic and k_shade, per traced ray for the traces.
 ADJ_DRAM_BYTES_PER_UNIT = {"k_logic (adjoint)": 378.8, "k_shade (adjoint)": 173.3,
                            "k_trace closest (extension)": 48.8, "k_trace any (shadow)": 93.7}
 # k_cache_infer: measured DRAM bytes per query (ncu over 6 cached 1080p
-# frames, 9,513,224 queries): the 64 B record in and the film update; the
+# frames, 9,513,228 queries): the 64 B record in and the film update; the
 # hash grid's FP16 copy stays in L2.
-CACHE_INFER_DRAM_BYTES_PER_QUERY = 110.8
+CACHE_INFER_DRAM_BYTES_PER_QUERY = 113.0
 # k_cache_infer's encoder: 16 levels x 8 corners x one 4-B FP16 pair per query.
 CACHE_GATHER_BYTES_PER_QUERY = 16 * 8 * 4
+
+
+def logic_bytes(per, hits, samples):
+    """k_logic's bytes for so many consumed hits and started samples."""
+    return per["hit"] * hits + per["vertex"] * max(0, hits - samples) + per["sample"] * samples
 
 
 def dist_env():
@@ -421,10 +433,10 @@ def l2_read_gbs(dev, mib=32, reps=40):
 
 # DRAM bytes per ray of k_trace launches, from an ncu capture at 4,194,304
 # rays per launch (the trace micro-benchmark's profile); traffic scales with rays.
-TRACE_DRAM_BYTES_PER_RAY = {"coherent_closest": (134.470144e6 + 42.339328e6) / 4194304,
-                            "incoherent_closest": (135.088384e6 + 40.223232e6) / 4194304,
-                            "coherent_any": (134.470144e6 + 42.339328e6) / 4194304,
-                            "incoherent_any": (135.088384e6 + 40.223232e6) / 4194304}
+TRACE_DRAM_BYTES_PER_RAY = {"coherent_closest": (134.410752e6 + 43.686144e6) / 4194304,
+                            "incoherent_closest": (135.150336e6 + 39.132416e6) / 4194304,
+                            "coherent_any": (134.404352e6 + 41.099264e6) / 4194304,
+                            "incoherent_any": (134.9888e6 + 38.324224e6) / 4194304}
 
 
 def reference_cuda_trace(scn, batches, d_hits):
@@ -724,8 +736,10 @@ def run_render(args, ws, rank, local, dist):
                                                         prof["extension_rays"] * WF_CLOSEST_BYTES,
                                                         f"{WF_CLOSEST_BYTES} B per extension ray (ray + tag in, "
                                                         "hit out)"),
-                 "k_logic": (prof["ms_logic"], prof["extension_rays"] * RENDER_LOGIC_BYTES_PER_HIT,
-                             f"{RENDER_LOGIC_BYTES_PER_HIT} B of slot state per consumed extension hit"),
+                 "k_logic": (prof["ms_logic"],
+                             logic_bytes(RENDER_LOGIC_BYTES, prof["extension_rays"], prof["samples"]),
+                             "{hit} B of slot state per consumed extension hit, {vertex} B per vertex, {sample} B per "
+                             "started sample".format(**RENDER_LOGIC_BYTES)),
                  "k_shade (all kinds)": (prof["ms_shade"], vertices * RENDER_SHADE_BYTES_PER_VERTEX
                                          + prof["shadow_rays"] * SHADOW_QUEUE_BYTES,
                                          f"{RENDER_SHADE_BYTES_PER_VERTEX} B of slot records and queue entries per "
@@ -901,7 +915,8 @@ def small_room_line(args, ws, rank, local, dist, ctx, dev, stream, steps=20, war
         stages = {"k_trace<any> (shadow queue)": (prof["ms_trace_shadow"], prof["shadow_rays"] * WF_ANY_BYTES),
                   "k_trace<closest> (extension queue)": (prof["ms_trace_extension"],
                                                          prof["extension_rays"] * WF_CLOSEST_BYTES),
-                  "k_logic": (prof["ms_logic"], prof["extension_rays"] * RENDER_LOGIC_BYTES_PER_HIT),
+                  "k_logic": (prof["ms_logic"],
+                              logic_bytes(RENDER_LOGIC_BYTES, prof["extension_rays"], prof["samples"])),
                   "k_shade (all kinds)": (prof["ms_shade"], max(0, prof["extension_rays"] - prof["samples"])
                                           * RENDER_SHADE_BYTES_PER_VERTEX + prof["shadow_rays"] * SHADOW_QUEUE_BYTES)}
         dom = max(stages, key=lambda n: stages[n][0])
@@ -1052,10 +1067,10 @@ def inverse_line(args, ws, rank, local, dist, ctx, dev, stream, known_lighting_r
         r["adjoint_rays"] = {"extension": ext_traced, "shadow": shadow_traced}
         dom = max(stages, key=stages.get)
         if dom.startswith("k_logic"):
-            # one consumed extension hit per slot and frame
-            achieved = ext_traced * ADJ_LOGIC_BYTES_PER_HIT / (stages[dom] / 1e3) / 1e9
-            note = (f"algorithmic bytes = {ADJ_LOGIC_BYTES_PER_HIT} B of slot state and records read and written per "
-                    "consumed extension hit over the stage's event-timed duration")
+            achieved = logic_bytes(ADJ_LOGIC_BYTES, ext_traced, prof["samples"]) / (stages[dom] / 1e3) / 1e9
+            note = ("algorithmic bytes = {hit} B of slot state per consumed extension hit, {vertex} B with its record "
+                    "per vertex and {sample} B per started sample over the stage's event-timed "
+                    "duration".format(**ADJ_LOGIC_BYTES))
         elif "trace" in dom:
             rays = ext_traced if "closest" in dom else shadow_traced
             per = WF_CLOSEST_BYTES if "closest" in dom else WF_ANY_BYTES

@@ -241,14 +241,13 @@ FF_D void load_costs(int32_t ref, float tri_area, const WidePlan* plan, float c[
     c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w, c[4] = b.x, c[5] = b.y, c[6] = b.z;
 }
 
-// The collapse that opened the child of largest area until 8 slots were used
-// gave 6.6 children a node on the small room; along the plan it is 7.5, and
-// incoherent rays fetch 2.6 instead of 3.3 nodes (closest hit), 1.6 instead
-// of 2.5 (any hit): 16.8M incoherent closest hits 1781 -> 1341 us, the 256 x
-// 256 x 16 render 2.87 -> 2.45 ms, the 1.3M-triangle 64-spp step 249.0 ->
-// 246.1 ms.  The DP runs where the bounds are formed, so the build's time
-// stays what it was (81,932 triangles under a sky: 10.0 and 9.8 ms to the
-// first hits).
+// Bounds bottom-up, and with them the plan of every subtree's collapse: both
+// need the children's and nothing else.  Bound by the climb, a chain of
+// dependent L2 accesses with a fence a level, in which 5 of 32 lanes take part
+// (82k triangles 66 us, 1.3M 269; the bounds alone 196).  What the plan gives:
+// against a collapse that opens the child of largest area until 8 slots are
+// used, incoherent rays in the small room fetch 2.6 instead of 3.3 nodes
+// (closest hit), 1.6 instead of 2.5 (any hit), 1,781 -> 1,341 us for 16.8M.
 __global__ void k_bounds_up(int n, const uint32_t* __restrict__ order, const float3* __restrict__ blo,
                             const float3* __restrict__ bhi, BinNode* nodes, WidePlan* plan,
                             const int32_t* __restrict__ parent_int, const int32_t* __restrict__ parent_leaf,

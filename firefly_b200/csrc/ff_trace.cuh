@@ -110,7 +110,8 @@ FF_D void ff_intersect_node(const FFNode8* __restrict__ nodes, uint32_t idx, con
     const float2 axy = make_float2(ax, ay), bxy = make_float2(bx, by), azz = make_float2(az, az),
                  bzz = make_float2(bz, bz);
     const float2 m23 = make_float2(-8388608.0f, -8388608.0f);
-    // meta bytes, four at a time: where an internal child (offset bits 24..31,
+    // meta bytes, four at a time (after Ylitie et al. 2017, "Efficient incoherent
+    // ray traversal on GPUs through compressed wide BVHs"): where an internal child (offset bits 24..31,
     // both upper bits set, which no leaf's offset has) or a leaf's triangles
     // go in the 32-bit answer, and the bits that go there (one bit for an
     // internal child, the unary count of a leaf, none for an empty slot, so

@@ -327,10 +327,9 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
     if (blockIdx.x == 0) {
         // the counters of frame + 2 start from zero, after their last frame's
         // rays join the totals; the host learns how many slots the last frame
-        // left active (with a launch of its own for the counters and a
-        // copy of the count that the host waited for every fourth frame, the 256
-        // x 256 preview took 639 us, so 501; 16 samples of it 2.24 and 2.15 ms, a
-        // 97 x 61 x 4 roughness adjoint 0.62 and 0.55 ms)
+        // left active.  (A small render is a chain of launches of tens of
+        // microseconds: a launch for the counters and a wait for the count
+        // every fourth frame made the 256 x 256 preview 639 us, this 501.)
         if (threadIdx.x < 2) w.totals[threadIdx.x] += w.ctr_next[threadIdx.x == 0 ? C_EXT : C_SH];
         if (threadIdx.x == 2 && !w.first) {
             w.progress[(w.frame - 1u) % kProgress] =
@@ -626,12 +625,9 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
     ff_ray ray{};
     if (push_ext) start_sample(w, s, sample, ray);
     // Compaction into the camera-ray part of the extension queue and the
-    // material queues, one atomic per block and queue.  Every counter sits in
-    // one L2 line, whose atomics run one after the other; with one atomic per
-    // warp and queue, and a 64-bit running total beside each, k_logic took
-    // 87.2 ms of the 1.3M-triangle 64-spp step, 76.9 ms so (with k_shade's
-    // single append per warp the step went from 259.7 to 249.0 ms, the small
-    // room's 256 x 256 x 16 from 3.06 to 2.87 ms).
+    // material queues, one atomic per block and queue: every counter sits in
+    // one L2 line, whose atomics run one after the other (one per warp and
+    // queue: 259.7 ms for the 1.3M-triangle 64-spp step, so 249.0).
     constexpr int kQ = kKinds + 2;   // the kinds, camera rays, active slots
     __shared__ uint32_t s_n[kLogicBlock / 32][kQ], s_base[kQ];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -687,8 +683,8 @@ __global__ void __launch_bounds__(kLogicBlock) k_logic(WF w)
 // during a replay.  CORR: corrected mode, whose reference lobes run in FP32
 // (parity mode keeps the reference's FP64 arithmetic; Lobes, ff_shade.cuh).
 // LK: what is known of the light (LightKind).  For the environment that
-// leaves 80 of the mix kind's 118 registers (6 instead of 4 blocks per SM),
-// for an area light 96.
+// leaves 92 of the mix kind's 122 registers (5 instead of 4 blocks per SM),
+// for an area light 102 (4); the diffuse kind's 89 become 56 and 80.
 template <int KIND, bool SEL, bool ADJ, bool CORR, int LK>
 __global__ void __launch_bounds__(128) k_shade(WF w)
 {
@@ -809,13 +805,9 @@ __global__ void __launch_bounds__(128) k_shade(WF w)
                     st_sector(&pq->b,
                               SlotMis{o.c_spec.x, o.c_spec.y, o.c_spec.z, 0.f, o.c_diff.x, o.c_diff.y, o.c_diff.z, 0.f});
                 // and the throughput after it in the place of the one before: 16
-                // bytes of a sector just read, where its factors took a record of
-                // 32 here and 32 more to read in k_logic.  With that, the sample
-                // counts derived from next_sample and no pass that clears the
-                // slots before the first frame, the 1.3M-triangle 64-spp step
-                // went from 234.4 to 230.5 ms, the inverse step (512 x 512 x 16)
-                // from 15.9 to 14.9 ms; more warps per SM (smaller blocks, fewer
-                // registers) change neither, so k_logic follows its bytes.
+                // bytes of a sector just read, where its factors would take a
+                // record of 32 here and 32 more to read in k_logic, whose time
+                // follows its bytes (more warps per SM change nothing).
                 const bool ends = path_ends(o.ext_f, o.ext_pdf);
                 float3 beta = xyz(beta_v);
                 if (!ends) beta *= (o.ext_f * o.ext_cos) / o.ext_pdf;
