@@ -440,25 +440,30 @@ __global__ void __launch_bounds__(kCollapseBlock)
             if (j) open(ref, j, i - j);
             else ch[nc++] = info(ref);
         }
-        // Where a box has no area (triangles on a line or in a point) or its
+        // Where the box has no area (triangles on a line or in a point) or its
         // area overflows (extents above 1e19), every split costs the same and
         // the plan has none: there the subtree with the most triangles is
         // opened until the slots are used, or the tree stays binary.
-        while (nc < 8) {
-            int most = -1;
-            uint32_t count = kLeafMax;
-            for (int c = 0; c < nc; ++c) {
-                const uint32_t cnt = ch[c].last - ch[c].first + 1;
-                const float a = half_area(ch[c].lo, ch[c].hi);
-                if (cnt > count && !(a > 0.f && a <= FLT_MAX)) {
-                    most = c;
-                    count = cnt;
+        auto costs = [](float3 lo, float3 hi) {
+            const float a = half_area(lo, hi);
+            return a > 0.f && a <= FLT_MAX;
+        };
+        if (!costs(bin[item.ref].lo, bin[item.ref].hi)) {
+            while (nc < 8) {
+                int most = -1;
+                uint32_t count = kLeafMax;
+                for (int c = 0; c < nc; ++c) {
+                    const uint32_t cnt = ch[c].last - ch[c].first + 1;
+                    if (cnt > count && !costs(ch[c].lo, ch[c].hi)) {
+                        most = c;
+                        count = cnt;
+                    }
                 }
+                if (most < 0) break;
+                const BinNode& b = bin[ch[most].ref];
+                ch[nc++] = info(b.right);
+                ch[most] = info(b.left);
             }
-            if (most < 0) break;
-            const BinNode& b = bin[ch[most].ref];
-            ch[nc++] = info(b.right);
-            ch[most] = info(b.left);
         }
     }
 
