@@ -178,6 +178,7 @@ SIGNATURES = {
     "ff_cache_write_params": (C.c_int, [P, P, P]),
     "ff_render_cached": (C.c_int, [P, P, P, C.POINTER(ff_render_settings), P, C.POINTER(ff_render_stats)]),
     "ff_debug_alloc_stats": (C.c_int, [C.POINTER(C.c_uint64), C.POINTER(C.c_int64)]),
+    "ff_debug_alloc_peak": (C.c_int, [C.POINTER(C.c_uint64)]),
     "ff_debug_fail_alloc_after": (C.c_int, [C.c_int64]),
     "ff_debug_trace_errors": (C.c_int, [P, C.c_uint32]),
     "ff_debug_cache_wait_limit": (C.c_int, [P, C.c_uint32]),

@@ -51,9 +51,14 @@ struct DeviceGuard {
     }
 };
 
-// One allocation for the scene's buffers, at the sizes the description gives.
-// (The tangent frames are allocated where a normal texture asks for them.)
-void place_scene(ff_scene* s, const ff_scene_desc* d)
+// One allocation for the scene's buffers, at the sizes the description gives,
+// where they come to at most kArenaMax.  A larger scene's are allocated as the
+// build comes to them: its 0.1 to 0.3 ms each are lost in the build, but
+// what is not there yet while the tree is built counts (80 of 168 bytes a
+// triangle, the textures, the environment).  (The tangent frames are allocated
+// where a normal texture asks for them.)
+constexpr size_t kArenaMax = 1ull << 30;
+void place_scene(ff_scene* s, const ff_scene_desc* d, bool together)
 {
     std::vector<std::pair<DevBuf*, size_t>> parts;
     const size_t n = d->num_triangles;
@@ -85,6 +90,7 @@ void place_scene(ff_scene* s, const ff_scene_desc* d)
     }
     size_t total = 0;
     for (auto& p : parts) total += (p.second + 255) & ~size_t(255);
+    if (!together || total > kArenaMax) return;
     s->arena.alloc(total);
     char* at = s->arena.as<char>();
     for (auto& p : parts) {
@@ -209,47 +215,55 @@ ff_status ff_scene_create(ff_context* ctx, const ff_scene_desc* d, ff_scene** ou
 {
     if (!ctx || !d || !out) return FF_ERR_INVALID_ARG;
     *out = nullptr;
-    ff_scene* s = new (std::nothrow) ff_scene();
-    if (!s) return FF_ERR_OOM;
-    s->ctx = ctx;
-    ff_status st = guarded(ctx, [&] {
-        DeviceGuard g(ctx->device);
-        FF_REQUIRE(d->num_triangles == 0 || (d->positions && d->indices), "positions and indices are required");
-        FF_REQUIRE(d->num_triangles == 0 || d->num_vertices > 0, "num_vertices must be > 0");
-        FF_REQUIRE(d->num_triangles < (1u << 30), "too many triangles");
-        uint32_t largest = 0;
-        for (uint64_t i = 0; i < 3ull * d->num_triangles; ++i) largest = std::max(largest, d->indices[i]);
-        FF_REQUIRE(d->num_triangles == 0 || largest < d->num_vertices, "triangle index out of range");
-        if (d->material_ids) {
-            largest = 0;
-            for (uint32_t i = 0; i < d->num_triangles; ++i) largest = std::max(largest, d->material_ids[i]);
-            FF_REQUIRE(d->num_triangles == 0 || largest < (d->num_materials ? d->num_materials : 1u),
-                       "material id out of range");
-        }
-        FF_REQUIRE(d->num_materials < (1u << 24), "at most 2^24 - 1 materials");
-        for (uint32_t m = 0; m < d->num_materials; ++m) {
-            const ff_material& mt = d->materials[m];
-            FF_REQUIRE(mt.kind >= FF_MAT_MIX && mt.kind <= FF_MAT_COAT, "unknown material kind");
-            if (mt.kind == FF_MAT_DIELECTRIC) s->refracts = true;
-            FF_REQUIRE(mt.base_color_tex < (int32_t)d->num_textures, "texture index out of range");
-            FF_REQUIRE(mt.roughness_tex < (int32_t)d->num_textures, "texture index out of range");
-        }
-        FF_REQUIRE(!d->env_rgb || (d->env_width > 0 && d->env_height > 0), "environment map has zero size");
-        FF_REQUIRE(d->num_area_lights == 0 || d->area_lights, "area_lights is NULL");
-        FF_REQUIRE(d->num_directional_lights == 0 || d->directional_lights, "directional_lights is NULL");
-        cudaStream_t stream = ctx->stream;
-        place_scene(s, d);
-        FFTemp temp(ctx);
-        float3* pos = temp.get<float3>(d->num_vertices);
-        uint3* idx = temp.get<uint3>(d->num_triangles);
-        if (pos) FF_CUDA_CHECK(cudaMemcpyAsync(pos, d->positions, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, stream));
-        if (idx) FF_CUDA_CHECK(cudaMemcpyAsync(idx, d->indices, sizeof(uint3) * d->num_triangles, cudaMemcpyHostToDevice, stream));
-        ff_build_bvh(ctx, s, pos, idx, d->num_triangles);
-        FF_REQUIRE(s->depth <= (uint32_t)kMaxStackDepth, "BVH deeper than the traversal stack");
-        ff_build_shading(ctx, s, d, pos, idx);
-        s->camera = d->camera;
-        FF_CUDA_CHECK(cudaStreamSynchronize(stream));
-    });
+    ff_scene* s = nullptr;
+    auto create = [&](bool together) {
+        s = new (std::nothrow) ff_scene();
+        if (!s) return FF_ERR_OOM;
+        s->ctx = ctx;
+        return guarded(ctx, [&] {
+            DeviceGuard g(ctx->device);
+            FF_REQUIRE(d->num_triangles == 0 || (d->positions && d->indices), "positions and indices are required");
+            FF_REQUIRE(d->num_triangles == 0 || d->num_vertices > 0, "num_vertices must be > 0");
+            FF_REQUIRE(d->num_triangles < (1u << 30), "too many triangles");
+            uint32_t largest = 0;
+            for (uint64_t i = 0; i < 3ull * d->num_triangles; ++i) largest = std::max(largest, d->indices[i]);
+            FF_REQUIRE(d->num_triangles == 0 || largest < d->num_vertices, "triangle index out of range");
+            if (d->material_ids) {
+                largest = 0;
+                for (uint32_t i = 0; i < d->num_triangles; ++i) largest = std::max(largest, d->material_ids[i]);
+                FF_REQUIRE(d->num_triangles == 0 || largest < (d->num_materials ? d->num_materials : 1u),
+                           "material id out of range");
+            }
+            FF_REQUIRE(d->num_materials < (1u << 24), "at most 2^24 - 1 materials");
+            for (uint32_t m = 0; m < d->num_materials; ++m) {
+                const ff_material& mt = d->materials[m];
+                FF_REQUIRE(mt.kind >= FF_MAT_MIX && mt.kind <= FF_MAT_COAT, "unknown material kind");
+                if (mt.kind == FF_MAT_DIELECTRIC) s->refracts = true;
+                FF_REQUIRE(mt.base_color_tex < (int32_t)d->num_textures, "texture index out of range");
+                FF_REQUIRE(mt.roughness_tex < (int32_t)d->num_textures, "texture index out of range");
+            }
+            FF_REQUIRE(!d->env_rgb || (d->env_width > 0 && d->env_height > 0), "environment map has zero size");
+            FF_REQUIRE(d->num_area_lights == 0 || d->area_lights, "area_lights is NULL");
+            FF_REQUIRE(d->num_directional_lights == 0 || d->directional_lights, "directional_lights is NULL");
+            cudaStream_t stream = ctx->stream;
+            place_scene(s, d, together);
+            FFTemp temp(ctx);
+            float3* pos = temp.get<float3>(d->num_vertices);
+            uint3* idx = temp.get<uint3>(d->num_triangles);
+            if (pos) FF_CUDA_CHECK(cudaMemcpyAsync(pos, d->positions, sizeof(float3) * d->num_vertices, cudaMemcpyHostToDevice, stream));
+            if (idx) FF_CUDA_CHECK(cudaMemcpyAsync(idx, d->indices, sizeof(uint3) * d->num_triangles, cudaMemcpyHostToDevice, stream));
+            ff_build_bvh(ctx, s, pos, idx, d->num_triangles);
+            FF_REQUIRE(s->depth <= (uint32_t)kMaxStackDepth, "BVH deeper than the traversal stack");
+            ff_build_shading(ctx, s, d, pos, idx);
+            s->camera = d->camera;
+            FF_CUDA_CHECK(cudaStreamSynchronize(stream));
+        });
+    };
+    ff_status st = create(true);
+    if (st == FF_ERR_OOM) {   // again with the least memory at a time
+        delete s;
+        st = create(false);
+    }
     if (st != FF_OK) {
         delete s;
         return st;
@@ -557,6 +571,13 @@ extern "C" ff_status ff_debug_alloc_stats(uint64_t* total, int64_t* live)
 {
     if (total) *total = g_ff_alloc.total.load();
     if (live) *live = g_ff_alloc.live.load();
+    return FF_OK;
+}
+
+extern "C" ff_status ff_debug_alloc_peak(uint64_t* bytes)
+{
+    const int64_t peak = g_ff_alloc.peak.exchange(g_ff_alloc.held.load());
+    if (bytes) *bytes = (uint64_t)peak;
     return FF_OK;
 }
 

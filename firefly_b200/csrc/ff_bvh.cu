@@ -660,14 +660,24 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
     FF_CUDA_CHECK(cudaEventRecord(e0, st));
 
     FFTemp temp(ctx);
+    const uint32_t n_int = n > 1 ? n - 1 : 1;
     FFTri* rec = temp.get<FFTri>(n);
     float3* blo = temp.get<float3>(n);
     float3* bhi = temp.get<float3>(n);
-    float3* cen = temp.get<float3>(n);
-    uint64_t* keys = temp.get<uint64_t>(n);
     uint64_t* keys2 = temp.get<uint64_t>(n);
-    uint32_t* vals = temp.get<uint32_t>(n);
     uint32_t* vals2 = temp.get<uint32_t>(n);
+    // what ends with the sort, and in its place the plans, which come after it
+    size_t sort_bytes = 0;
+    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (uint64_t*)nullptr, keys2, (uint32_t*)nullptr,
+                                                  vals2, (int)n, 0, 64, st));
+    const size_t pad = 255, at_keys = (sizeof(float3) * (size_t)n + pad) & ~pad,
+                 at_vals = at_keys + ((sizeof(uint64_t) * (size_t)n + pad) & ~pad),
+                 at_sort = at_vals + ((sizeof(uint32_t) * (size_t)n + pad) & ~pad);
+    char* early = temp.get<char>(std::max(at_sort + std::max<size_t>(sort_bytes, 16), sizeof(WidePlan) * n_int));
+    float3* cen = reinterpret_cast<float3*>(early);
+    uint64_t* keys = reinterpret_cast<uint64_t*>(early + at_keys);
+    uint32_t* vals = reinterpret_cast<uint32_t*>(early + at_vals);
+    WidePlan* plan = reinterpret_cast<WidePlan*>(early);
     uint32_t* counters = temp.get<uint32_t>(64 + kMaxLevels + 1);
     uint32_t* level = counters + 64;
     int* cb = reinterpret_cast<int*>(counters + 16);
@@ -679,18 +689,12 @@ void ff_build_bvh(ff_context* ctx, ff_scene* s, const float3* d_pos, const uint3
                             cen, cb, cb + 12);
     k_morton<<<G, B, 0, st>>>(cen, n, cb, keys, vals, blo,
                               bhi);
-    size_t temp_bytes = 0;
-    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys2,
-                                                  vals, vals2, (int)n, 0, 64, st));
-    void* sort_temp = temp.get<char>(std::max<size_t>(temp_bytes, 16));
-    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_temp, temp_bytes, keys, keys2,
+    FF_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(early + at_sort, sort_bytes, keys, keys2,
                                                   vals, vals2, (int)n, 0, 64, st));
     const uint64_t* skeys = keys2;
     const uint32_t* order = vals2;
 
-    uint32_t n_int = n > 1 ? n - 1 : 1;
     BinNode* bin = temp.get<BinNode>(n_int);
-    WidePlan* plan = temp.get<WidePlan>(n_int);
     int32_t* pint = temp.get<int32_t>(n_int);
     int32_t* pleaf = temp.get<int32_t>(n);
     uint32_t* arrivals = temp.get<uint32_t>(n_int);

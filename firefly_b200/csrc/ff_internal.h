@@ -4,7 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -35,14 +37,21 @@ struct FFError {
         if (!(cond)) throw FFError{FF_ERR_INVALID_ARG, (msg)}; \
     } while (0)
 
-// Device allocations made through DevBuf, process-wide (ff_debug_alloc_stats),
-// and the test hook that refuses them (ff_debug_fail_alloc_after): while
+// Device allocations made through DevBuf, process-wide (ff_debug_alloc_stats,
+// ff_debug_alloc_peak), and the test hook that refuses them (ff_debug_fail_alloc_after): while
 // fail_after >= 0, that many more allocations succeed and every later one
 // fails with FF_ERR_OOM without reaching cudaMalloc.
 struct FFAllocStats {
     std::atomic<uint64_t> total{0};
     std::atomic<int64_t> live{0};
     std::atomic<int64_t> fail_after{-1};
+    std::atomic<int64_t> held{0}, peak{0};   // bytes now, and the most since peak was last set to held
+    void hold(int64_t bytes)
+    {
+        const int64_t now = held.fetch_add(bytes) + bytes;
+        int64_t most = peak.load();
+        while (now > most && !peak.compare_exchange_weak(most, now)) {}
+    }
 };
 extern FFAllocStats g_ff_alloc;
 
@@ -84,6 +93,7 @@ struct DevBuf {
         if (ptr && owned) {
             cudaFree(ptr);
             g_ff_alloc.live.fetch_sub(1);
+            g_ff_alloc.hold(-(int64_t)bytes);
         }
         ptr = nullptr;
         bytes = 0;
@@ -115,6 +125,7 @@ struct DevBuf {
         }
         g_ff_alloc.total.fetch_add(1);
         g_ff_alloc.live.fetch_add(1);
+        g_ff_alloc.hold((int64_t)n);
         bytes = n;
     }
     template <class T>
@@ -122,7 +133,9 @@ struct DevBuf {
 };
 
 // Device memory for the temporaries of calls on one context, in blocks handed
-// out from the front and taken back together (FFTemp).  A cudaMalloc and
+// out from the front and taken back together (FFTemp).  An inner scope's blocks
+// go back at its end once there are more than kKeep bytes, so that a large
+// build's temporaries are not held beside those of the shading data.  A cudaMalloc and
 // cudaFree cost 0.1 to 0.3 ms each and the free waits for the device: 35 of
 // both were over 80% of a scene's load (81,932 triangles under a 1024 x 512
 // sky: 9.8 ms, now 2.4).  Between calls one block of at most kKeep bytes stays; the
@@ -145,25 +158,33 @@ struct FFScratch {
     {
         n = (n + 255) & ~size_t(255);
         if (blocks.empty() || used + n > blocks.back()->bytes) {
-            DevBuf* b = new DevBuf();
+            blocks.reserve(blocks.size() + 1);
+            std::unique_ptr<DevBuf> b(new DevBuf());
             try {
-                b->alloc(n > next_min ? n : next_min);
-                blocks.push_back(b);
-            } catch (...) {
-                delete b;
-                throw;
+                b->alloc(std::max(n, next_min));
+            } catch (const FFError& e) {
+                if (e.status != FF_ERR_OOM || n >= next_min) throw;
+                b->alloc(n);   // a nearly full device
             }
+            blocks.push_back(b.release());
             used = 0;
         }
         void* p = static_cast<char*>(blocks.back()->ptr) + used;
         used += n;
         return p;
     }
-    void close_scope()
+    // A scope that began with `first` blocks, the last used up to `at`, ends.
+    void close_scope(size_t first, size_t at)
     {
-        if (--scopes) return;
+        --scopes;
         size_t total = 0;
         for (DevBuf* b : blocks) total += b->bytes;
+        if (scopes) {
+            if (total <= kKeep) return;
+            for (; blocks.size() > first; blocks.pop_back()) delete blocks.back();
+            used = at;
+            return;
+        }
         if (blocks.size() > 1 || total > kKeep) {   // one block for the next call of this size
             release();
             next_min = total > kKeep ? kMinBlock : total;
@@ -265,8 +286,9 @@ struct FFEnvLight {
 // Temporaries of one call on the context's stream, given back at scope end.
 struct FFTemp {
     FFScratch& s;
-    explicit FFTemp(ff_context* ctx) : s(ctx->scratch) { ++s.scopes; }
-    ~FFTemp() { s.close_scope(); }
+    const size_t first, at;
+    explicit FFTemp(ff_context* ctx) : s(ctx->scratch), first(s.blocks.size()), at(s.used) { ++s.scopes; }
+    ~FFTemp() { s.close_scope(first, at); }
     FFTemp(const FFTemp&) = delete;
     FFTemp& operator=(const FFTemp&) = delete;
     template <class T>
@@ -275,7 +297,7 @@ struct FFTemp {
 
 struct ff_scene {
     ff_context* ctx = nullptr;
-    DevBuf arena;         // the buffers below whose sizes the description gives sit in it
+    DevBuf arena;         // the buffers below whose sizes the description gives sit in it (place_scene)
     uint32_t num_tris = 0;
     uint32_t num_nodes = 0;
     uint32_t depth = 0;

@@ -162,7 +162,8 @@ void ff_build_shading(ff_context* ctx, ff_scene* s, const ff_scene_desc* d, cons
         for (uint32_t i = 0; i < d->num_textures; ++i) {
             const ff_texture_desc& td = d->textures[i];
             FF_REQUIRE(td.rgb && td.width > 0 && td.height > 0, "texture without texels");
-            DevBuf* b = s->textures[i];   // (placed at creation)
+            DevBuf* b = s->textures[i];
+            b->alloc(sizeof(float3) * td.width * td.height);   // (where it was not placed at creation)
             FF_CUDA_CHECK(cudaMemcpyAsync(b->ptr, td.rgb, sizeof(float3) * td.width * td.height, cudaMemcpyHostToDevice, st));
             views[i] = FFTexView{b->as<float3>(), (int)td.width, (int)td.height};
         }

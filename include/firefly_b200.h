@@ -515,6 +515,10 @@ FF_API ff_status ff_render_cached(ff_context* ctx, ff_scene* scene, ff_cache* ca
 /* Device allocations this library made since it was loaded (total) and the
  * ones it still holds (live), over all contexts.  Either pointer may be NULL. */
 FF_API ff_status ff_debug_alloc_stats(uint64_t* total, int64_t* live);
+/* The most bytes of device memory that this library's allocations came to at
+ * once since the last call of this hook (or since it was loaded), over all contexts.
+ * bytes may be NULL. */
+FF_API ff_status ff_debug_alloc_peak(uint64_t* bytes);
 /* From now on the next n device allocations of this library succeed and
  * every later one fails with FF_ERR_OOM, without calling cudaMalloc; n < 0
  * turns the refusal off.  Process-wide. */
