@@ -693,7 +693,13 @@ void ff_cache_setup_grid(ff_cache* c)
         total += n;
         g.cell_levels = (uint32_t)l + 1u;
     }
-    c->cells.alloc(32 * total);
+    // (a copy: a device without the room for it gets the same answers from the table)
+    try {
+        c->cells.alloc(32 * total);
+    } catch (const FFError& e) {
+        if (e.status != FF_ERR_OOM) throw;
+        g.cell_levels = 0;
+    }
     g.cells = c->cells.as<uint4>();
 }
 
